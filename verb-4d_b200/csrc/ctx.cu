@@ -228,6 +228,7 @@ int local_prepare(verb_ctx* c, LocalArgs& a, double dts)
     a.kvp32 = c->kvp32;
     a.Lf32 = c->Lf32;
     a.Uf32 = c->Uf32;
+    a.unknowns = nu;
     a.ipiv = c->ipiv;
     a.k0 = c->trim_k0;
     a.uoff = c->trim_uoff;
@@ -260,11 +261,6 @@ int local_factor(verb_ctx* c, LocalArgs& a)
 {
     CK(alloc_factors(c, a));
     PhaseTimer t(c, PH_LOCF);
-    const size_t nu = c->local_unknowns;
-    if (a.factors32)
-        CK(cudaMemsetAsync(c->Uf32, 0, nu * c->kvp32 * sizeof(float), c->stream));
-    else
-        CK(cudaMemsetAsync(c->Uf, 0, nu * c->kvp * sizeof(double), c->stream));
     c->acc.kernel_launches += launch_local_factor(a, c->stream);
     c->local_dirty = false;
     c->local_dt = a.dt;

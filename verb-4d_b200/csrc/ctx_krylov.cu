@@ -175,11 +175,6 @@ int krylov_run(verb_ctx* c, double dt, double sub_dt, int guess, verb_cnn* cnn, 
             ap.sel_mask = 3;
             s = alloc_factors(c, ap);
             if (s) return s;
-            const size_t nuf = c->local_unknowns;
-            if (ap.factors32)
-                CK(cudaMemsetAsync(c->Uf32, 0, nuf * c->kvp32 * sizeof(float), c->stream));
-            else
-                CK(cudaMemsetAsync(c->Uf, 0, nuf * c->kvp * sizeof(double), c->stream));
             c->acc.kernel_launches += launch_local_factor(ap, c->stream);
             launch_local_solve(ap, c->stream);
             c->acc.kernel_launches++;

@@ -10,7 +10,8 @@
 // coefficients change (src/VERB4D_Solver.cpp:1091-1096).
 //
 // Kernels:
-//  * local_factor_kernel: one CTA per system.  Rows of A are assembled on the
+//  * local_factor_kernel: one CTA per system (V < 7 and grids of more than
+//    65535 systems).  Rows of A are assembled on the
 //    device with the reference's operation order (bit-identical matrix) and
 //    factored by the unblocked banded LU of LAPACK's xGBTF2 (partial pivoting,
 //    multipliers scaled by the reciprocal pivot, rank-1 updates as fused
@@ -18,11 +19,11 @@
 //    The active (kl+1) x (kv+1) window lives in shared memory as a circular
 //    buffer over rows and columns.  Output: L multipliers (Lf, column j
 //    contiguous), U columns (Uf, rows j-kv..j contiguous) and 0-based pivots.
-//  * local_rows_kernel + local_factor_rw_kernel: the same factorisation with
-//    the window in registers (eight warps, bands up to V = 110): the rows are
-//    assembled beforehand and parked in the L columns they precede, and
-//    stream into a shared-memory ring by cp.async.  local_factor_kernel is
-//    kept for wider bands.
+//  * local_rows_kernel + local_factor_blk_kernel: the same factorisation by
+//    panels of columns, for every other grid: the rows are assembled
+//    beforehand and parked in the L columns they precede, a panel's pivot
+//    chain and the update by the previous panel run side by side, and the
+//    update is on the FP64 matrix instruction.
 //  * local_rhs_kernel / local_store_kernel: tile transposes between the PSD
 //    slab [V][K] and the unknown order, forming RHS = B o f + C.
 //  * local_solve_kernel: one warp per system, the forward (L, interleaved row
@@ -39,6 +40,8 @@
 // as one fused multiply-add per element (fma()), so factors, pivots and
 // solutions are bit-identical to it.
 #include "verb_internal.cuh"
+
+#include <type_traits>
 
 namespace verb {
 
@@ -367,72 +370,11 @@ __global__ void __launch_bounds__(FACT_THREADS) local_factor_kernel(LocalArgs a)
     }
 }
 
-// The same factorisation with the (kl+1) x (kv+1) circular window held in
-// registers for the whole run.  NW warps (eight in use); warp w owns row slots
-// w + NW q (q < NR), lane l column slots l + 32 k (k < NC), value R[q][k].  Per column
-// j there are two block barriers:
-//   top   the lanes that own column slot j % CW search their own rows for the
-//         first maximum of |x| (they updated those values themselves at
-//         column j-1, so no barrier is needed before the search) and post the
-//         column and their warp's candidate;
-//   B1    every thread combines the NW candidates (idamax: first maximum,
-//         NaN skipped unless it is the first entry); the multipliers go to
-//         Lf; every thread forms one window slot of the row that enters at
-//         the next column; the owners of row j and of the pivot row post them;
-//   B2    the swap over columns j..ju in the owners' registers, U row j out,
-//         the rank-1 update of every owned slot (multipliers from the posted
-//         column, the pivot row from shared memory), and the slide: column
-//         slot j % CW is cleared, row slot j % RW takes row j+kl+1 (formed at
-//         the previous column).
-// The row and column slots of the pivot step are reached through a switch on
-// their index (registers cannot be indexed at run time), so only the rank-1
-// update touches every slot.  Every element sees the same operations in the
-// same order as in local_factor_kernel (LAPACK's xGBTF2, the rank-1 update
-// fused): factors and pivots are bit-identical, and the update costs no
-// shared-memory traffic.
-// f(R[q]) for a run-time q < NR
-template <int NR, int NC, typename F>
-__device__ __forceinline__ void frw_row(double (&R)[NR][NC], int q, F&& f)
-{
-    switch (q) {
-#define VERB_ROW(Q) \
-    case Q:         \
-        if constexpr (Q < NR) f(R[Q]); \
-        break;
-        VERB_ROW(0) VERB_ROW(1) VERB_ROW(2) VERB_ROW(3) VERB_ROW(4) VERB_ROW(5) VERB_ROW(6)
-        VERB_ROW(7) VERB_ROW(8) VERB_ROW(9) VERB_ROW(10) VERB_ROW(11) VERB_ROW(12) VERB_ROW(13)
-#undef VERB_ROW
-        default: break;
-    }
-}
-
-template <int K, int NR, int NC, typename F>
-__device__ __forceinline__ void frw_col_k(double (&R)[NR][NC], F& f)
-{
-#pragma unroll
-    for (int q = 0; q < NR; q++) f(q, R[q][K]);
-}
-
-// f(q, R[q][k]) for every q, for a run-time k < NC
-template <int NR, int NC, typename F>
-__device__ __forceinline__ void frw_col(double (&R)[NR][NC], int k, F&& f)
-{
-    switch (k) {
-#define VERB_COL(K) \
-    case K:         \
-        if constexpr (K < NC) frw_col_k<K>(R, f); \
-        break;
-        VERB_COL(0) VERB_COL(1) VERB_COL(2) VERB_COL(3) VERB_COL(4) VERB_COL(5) VERB_COL(6)
-#undef VERB_COL
-        default: break;
-    }
-}
-
 // Every row of A, assembled once before the factorisation and parked in the
 // L-factor column of the same index: row q's nine diagonal values go to
-// Lf[q][0..8] (as FP64, also when the factors are FP32).  local_factor_rw_kernel
-// reads row q at column q-kl-1 (or for the first window) and writes L column q
-// only at column q, so the parked row is always read before it is overwritten.
+// Lf[q][0..8] (as FP64, also when the factors are FP32).  local_factor_blk_kernel
+// reads row q at least kl columns before it (or for the first window) and writes
+// L column q only in the panel of column q, so the parked row is always read before it is overwritten.
 template <typename T>
 __device__ __forceinline__ double* frw_row_slot(const LocalArgs& a, size_t u)
 {
@@ -466,239 +408,558 @@ __device__ __forceinline__ void cp_async_8(double* dst, const double* src)
 __device__ __forceinline__ void frw_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void frw_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-template <typename T, int NR, int NC, int NW>
-__global__ void __launch_bounds__(NW * 32, 1) local_factor_rw_kernel(LocalArgs a)
+// Blocked form of the same factorisation.  Columns are taken NB at a time: PW
+// warps factor the panel (the NB columns over the kl + NB rows they reach) in
+// registers, one row a thread; the other warps meanwhile
+// apply the previous panel to the columns right of it, so the pivot chain of
+// the next panel and the multiply-adds of this one run at the same time.  The
+// (kl + NB) x (kv + NB) window lives in shared memory, circular in rows and
+// columns.  The update is a product over the NB pivots on the FP64 matrix
+// instruction (m8n8k4): a warp keeps the multipliers of 16 rows in registers
+// and runs along the columns, so an element is loaded and stored once per NB
+// columns.
+//
+// Every element sees the operations of local_factor_kernel (LAPACK's xGBTF2
+// with the rank-1 update fused) in the same order: the update of element
+// (i, c) by pivot k is fma(l_ik, -u_kc, a_ic), pivots in ascending order (the
+// matrix instruction adds its four products one fused multiply-add at a time
+// in that order: bit-equal to the fma chain), and a row's multipliers move
+// with the row when a later pivot of the panel interchanges it.  Factors and
+// pivots are therefore bit-identical to it.  xGBTF2 skips the update where
+// u_kc = 0; adding a zero product leaves a finite element as it is, so the
+// skip is only taken where a panel holds a zero or tiny pivot or a value that
+// is not finite (the slow branches below).
+//
+// 24 x 51 x 101 x 21 (1224 systems, factors 12.9 GB): 55 ms for the unblocked
+// register-window kernel this replaces, 13.5 ms here; 24 x 25 x 31 x 31, the
+// mixed form's whole pass: 4.76 -> 1.98 ms.  The bound is the panel: about
+// 1000 cycles a column of pivot search and exchange through shared memory,
+// against 160-320 for the multiply-adds of the update, which run beside it,
+// and 4 of the 13.5 ms for writing the factors at the copy bandwidth.
+constexpr int NB = 8;  // columns of a panel
+
+struct FBlk {
+    int RW, CW, pitch;  // window rows, columns, row pitch in doubles
+};
+
+__device__ __forceinline__ void named_sync(int id, int threads)
 {
-    extern __shared__ double sm[];
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// c (8 x 8: row lane / 4, columns 2 (lane % 4), + 1) += a (8 x 4: row lane / 4,
+// column lane % 4) times b (4 x 8: row lane % 4, column lane / 4)
+__device__ __forceinline__ void dmma(double2& c, double a, double b)
+{
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+        : "+d"(c.x), "+d"(c.y)
+        : "d"(a), "d"(b));
+}
+
+// RN(1 / x) for 2^-1000 < |x| < 2^1000: Newton steps from the hardware's
+// approximation, the last one correcting by the exact residual, which rounds
+// correctly except where the significand of x is all ones (Markstein, IBM J.
+// Res. Dev. 34, 1990); there 1/x lies just above the midpoint of a power of
+// two and its successor and rounds to the successor.  Without a division's
+// range branch the steps interleave with the pivot search.
+__device__ __forceinline__ double recip(double x)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+#pragma unroll
+    for (int i = 0; i < 4; i++) y = fma(y, fma(-x, y, 1.0), y);
+    const long long ones = 0xfffffffffffffLL;
+    const bool all = (__double_as_longlong(x) & ones) == ones;
+    return all ? __longlong_as_double(__double_as_longlong(y) | 1) : y;
+}
+
+// *p = (x, y) in shared memory where c holds, as a predicated store
+__device__ __forceinline__ void sts2_if(bool c, double* p, double x, double y)
+{
+    asm volatile(
+        "{\n .reg .pred q;\n setp.ne.s32 q, %0, 0;\n @q st.shared.v2.f64 [%1], {%2, %3};\n}" ::"r"(
+            (int)c),
+        "r"((unsigned)__cvta_generic_to_shared(p)), "d"(x), "d"(y)
+        : "memory");
+}
+
+template <typename T, int PW, int NW>
+__global__ void __launch_bounds__(NW * 32) local_factor_blk_kernel(LocalArgs a, FBlk f)
+{
+    extern __shared__ __align__(16) double sm[];
     const int sys = blockIdx.x;
     if (skip_system(a, sys)) return;
     const int nx = a.d.V;
     const int n = a.d.V * (a.d.K - sys_k0(a, sys));
     const size_t u0 = sys_uoff(a, sys);
     const int kl = a.kl, ku = a.kl, kv = a.kv;
-    const int RW = kl + 1;          // window rows
-    const int CW = kv + 1;          // window columns
-    double* stage = sm;             // [2 STAGE_ROWS][9] ring of parked rows
-    double* rowA = stage + (size_t)2 * STAGE_ROWS * 9;  // [CW] row j before the swap
-    double* rowB = rowA + CW;       // [CW] the pivot row (row j after the swap)
-    double* colv = rowB + CW;       // [2][RW] column j by offset, by parity of j
-    double* nrow = colv + 2 * RW;   // [2][CW] the window row that enters at column j, by parity
-    __shared__ double s_best[NW];
-    __shared__ int s_bi[NW];
+    const int RW = f.RW, CW = f.CW, pitch = f.pitch;
+    double* W = sm;                                // [RW][pitch]
+    double* stage = W + (size_t)RW * pitch;        // [2][NB][10] entering rows
+    double* newp = stage + 2 * NB * 10;            // [NB][NB] their part in the next panel
+    double* prow = newp + NB * NB;                 // [2][PW][NB+4] pivot candidates of the warps
+    double* tri = prow + 2 * PW * (NB + 4);                   // [2][NB][NB] multipliers within a panel, negated
+    // a panel's interchanges as one permutation of the rows (window offsets):
+    // row k <- row s_src[k], and s_no rows below the panel <- rows of it
+    __shared__ int s_src[2][NB], s_od[2][NB], s_os[2][NB], s_no[2];
+    __shared__ int s_ju[2];                        // last column a panel's pivot rows reach
+    __shared__ int s_bad[2];                       // a non-finite multiplier in the panel
+    __shared__ int s_badu;                         // a non-finite U entry
+    __shared__ int s_huge;                         // a value above 2^1000 in the panel
     const bool f32 = sizeof(T) == sizeof(float);
     const int klp = f32 ? a.klp32 : a.klp, kvp = f32 ? a.kvp32 : a.kvp;
     T* Lf = (f32 ? (T*)a.Lf32 : (T*)a.Lf) + u0 * klp;
     T* Uf = (f32 ? (T*)a.Uf32 : (T*)a.Uf) + u0 * kvp;
     int32_t* ip = a.ipiv + u0;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-
-    // rows 256 b .. 256 b + 255 (parked by local_rows_kernel) into ring half
-    // b % 2, asynchronously
     const double* rows = frw_row_slot<T>(a, u0);
     const size_t rstride = f32 ? (size_t)a.klp32 / 2 : (size_t)a.klp;  // doubles
-    auto fetch_block = [&](int b) {
-        const int q0 = b * STAGE_ROWS;
-        const int cnt = min(STAGE_ROWS, n - q0) * 9;
-        for (int e = tid; e < cnt; e += blockDim.x) {
-            const int q = q0 + e / 9, s2 = e - (e / 9) * 9;
-            cp_async_8(stage + (size_t)(q & (2 * STAGE_ROWS - 1)) * 9 + s2, rows + q * rstride + s2);
+
+    // column offset of the nine stored diagonals
+    auto diag_off = [&](int s) { return (s / 3 - 1) * nx + (s % 3 - 1); };
+    // the rows that enter when the panel at j0 is done
+    auto fetch_rows = [&](int j0, int buf, int t, int nt) {
+        for (int e = t; e < NB * 9; e += nt) {
+            const int r = e / 9, s = e - r * 9, q = j0 + RW + r;
+            if (q < n) cp_async_8(stage + (buf * NB + r) * 10 + s, rows + q * rstride + s);
         }
         frw_commit();
     };
-    auto row_value = [&](int q, int col) -> double {
-        const int d = col - q;
-        const int dy = (d < -1) ? -1 : (d > 1 ? 1 : 0);
-        const int dx = d - dy * nx;
-        if (dx < -1 || dx > 1 || col < 0 || col >= n) return 0.0;
-        return stage[(q & (2 * STAGE_ROWS - 1)) * 9 + dslot(dx, dy)];
-    };
 
-    double R[NR][NC];
-    fetch_block(0);
-    if (n > STAGE_ROWS) fetch_block(1);
-    frw_wait_all();
+    // first window: rows 0 .. RW-1; the U entries above row 0 are zero
+    for (int e = tid; e < RW * pitch; e += NW * 32) W[e] = 0.0;
+    for (int c = wid; c < min(kv, n); c += NW)
+        for (int q = lane; q < kv - c; q += 32) Uf[(size_t)c * kvp + q] = (T)0;
+    if (tid == 0) s_badu = 0;
     __syncthreads();
-    // the row entering at column jj (row jj+kl+1) over window slots: slot cs
-    // holds column jj+1+((cs-(jj+1)) mod CW); cjj = jj mod CW
-    auto fill_row = [&](int jj, int cjj) {
-        const int qr = jj + kl + 1;
-        for (int cs = tid; cs < CW; cs += blockDim.x) {
-            int c = cs - cjj - 1;
-            if (c < 0) c += CW;
-            nrow[(jj & 1) * CW + cs] = qr < n ? row_value(qr, jj + 1 + c) : 0.0;
+    for (int e = tid; e < min(RW, n) * 9; e += NW * 32) {
+        const int q = e / 9, s = e - q * 9, c = q + diag_off(s);
+        if (c >= 0 && c < n) W[q * pitch + c] = rows[q * rstride + s];
+    }
+    __syncthreads();
+
+    // One panel: columns j0 .. j0+NB-1 over rows j0 .. j0+RW-1, row tid of
+    // them by each thread of the first PW warps; rj, cj: window slots of row
+    // and column j0.  first: every row is in the window, else the last NB ones
+    // are in newp.  Returns the new ju.  What a column costs is the chain from
+    // its updated values through the pivot search to the next update, and the
+    // instructions the warps fetch on the way: the loop stays rolled (column
+    // jj is always R[0]; the update writes column c to R[c-1], the finished
+    // column goes to the end), rows are not interchanged in the registers,
+    // only their positions pos are, and there is one barrier a column.
+    auto panel = [&](int j0, int rj, int cj, int par, bool first, int ju) {
+        constexpr int PT = PW * 32;
+        double R[NB];
+        const int t = tid, nbk = min(NB, n - j0);
+        int pos = t;
+        auto slot = [&](int c) { return cj + c < CW ? cj + c : cj + c - CW; };
+        auto off = [&](int i) { return (rj + i < RW ? rj + i : rj + i - RW) * pitch; };
+        unsigned top = 0;
+        {
+            const bool win = first || t < kl;
+            const double* src = win ? W + off(t) : newp + (t - kl) * NB;
+#pragma unroll
+            for (int c = 0; c < NB; c += 2) {
+                double2 v = make_double2(0.0, 0.0);
+                if (t < RW) v = *(const double2*)(src + (win ? slot(c) : c));
+                R[c] = v.x;
+                R[c + 1] = v.y;
+                top = max(top, max((unsigned)__double2hiint(v.x) & 0x7fffffffu,
+                                   (unsigned)__double2hiint(v.y) & 0x7fffffffu));
+            }
         }
+        // values up to 2^1000 stay finite over a panel (|l| <= 1); larger ones
+        // and pivots whose reciprocal overflows take the slow branch
+        if (tid == 0) {
+            s_no[par] = 0;
+            s_huge = 0;
+        }
+        named_sync(2, PT);
+        if (top >= 0x7e700000u) s_huge = 1;
+        int jj = 0;
+        T* pl = Lf + (size_t)j0 * klp - 1;
+#pragma unroll 1
+        for (; jj < nbk; jj++) {
+            // the warp's first maximum of |column jj| over positions jj ..
+            // jj+kl, by the upper words, the lower ones only where those tie
+            const int last = min(jj + kl, n - 1 - j0);
+            const unsigned h =
+                pos >= jj && pos <= last ? (unsigned)__double2hiint(R[0]) & 0x7fffffffu : 0u;
+            const unsigned wh = __reduce_max_sync(0xffffffffu, h);
+            const double rinv = recip(R[0]);
+            bool own = h == wh;
+            const unsigned b = __ballot_sync(0xffffffffu, own);
+            if (b & (b - 1)) {
+                const unsigned lo = own && wh ? (unsigned)__double2loint(R[0]) : 0u;
+                const unsigned wl = __reduce_max_sync(0xffffffffu, lo);
+                own = own && lo == wl;
+                const unsigned p = own ? pos : 1u << 20;
+                own = p == __reduce_min_sync(0xffffffffu, p);
+            }
+            // its row, reciprocal, |pivot| and position
+            double* cand = prow + ((jj & 1) * PW + wid) * (NB + 4);
+#pragma unroll
+            for (int c = 0; c < NB; c += 2) sts2_if(own, cand + c, R[c], R[c + 1]);
+            sts2_if(own, cand + NB, wh ? fabs(R[0]) : 0.0, __hiloint2double(0, wh ? pos : 1 << 20));
+            sts2_if(own, cand + NB + 2, rinv, 0.0);
+            named_sync(2, PT);
+            const double* best = prow + (jj & 1) * PW * (NB + 4);
+            double2 key = *(const double2*)(best + NB);
+#pragma unroll
+            for (int w = 1; w < PW; w++) {
+                const double* o = prow + ((jj & 1) * PW + w) * (NB + 4);
+                const double2 k = *(const double2*)(o + NB);
+                const long long ka = __double_as_longlong(k.x), kb = __double_as_longlong(key.x);
+                if (ka > kb || (ka == kb && __double2loint(k.y) < __double2loint(key.y))) {
+                    key = k;
+                    best = o;
+                }
+            }
+            if (s_huge || __double2hiint(key.x) < 0x00400000) break;
+            const int tp = __double2loint(key.y);
+            double uc[NB];
+#pragma unroll
+            for (int c = 0; c < NB; c += 2) {
+                const double2 v = *(const double2*)(best + c);
+                // finished columns sit at the end: no update
+                uc[c] = c < NB - jj ? -v.x : 0.0;
+                uc[c + 1] = c + 1 < NB - jj ? -v.y : 0.0;
+            }
+            const double rcp = best[NB + 2];
+            if (tid == 0) ip[j0 + jj] = j0 + tp;
+            ju = max(ju, min(j0 + ku + tp, n - 1));
+            pos = pos == tp ? jj : (pos == jj ? tp : pos);
+            const double m = R[0] * rcp;
+            const bool act = pos > jj && pos <= last;
+            if (act) pl[pos] = (T)m;
+            const double l = act ? m : 0.0, fin = act ? m : R[0];
+#pragma unroll
+            for (int c = 1; c < NB; c++) R[c - 1] = fma(l, uc[c], R[c]);
+            R[NB - 1] = fin;
+            pl += klp - 1;
+        }
+        // the panel back into the window, every row at its position
+        const bool bad = jj < nbk;
+        if (jj == NB) {
+            double* row = W + off(pos);
+            if (t < RW)
+#pragma unroll
+                for (int c = 0; c < NB; c += 2)
+                    *(double2*)(row + slot(c)) = make_double2(R[c], R[c + 1]);
+        } else {
+            // R[c] is column jj + c, the finished ones follow from the start
+#pragma unroll 1
+            for (int c = 0; c < NB; c++) {
+                if (t < RW) W[off(pos) + slot((jj + c) % NB)] = R[0];
+#pragma unroll
+                for (int k = 1; k < NB; k++) R[k - 1] = R[k];
+            }
+        }
+        named_sync(2, PT);
+        if (bad) {
+            // the rest of the panel in the window, operation by operation as
+            // xGBTF2 does it
+            auto at = [&](int i, int c) -> double& { return W[off(i) + slot(c)]; };
+#pragma unroll 1
+            for (; jj < nbk; jj++) {
+                const int j = j0 + jj, km = min(kl, n - 1 - j);
+                int p = jj;
+                double best = fabs(at(jj, jj));
+#pragma unroll 1
+                for (int i = jj + 1; i <= jj + km; i++) {
+                    const double v = fabs(at(i, jj));
+                    if (v > best) {
+                        best = v;
+                        p = i;
+                    }
+                }
+                const double piv = at(p, jj);
+                const bool nz = piv != 0.0;
+                if (nz) ju = max(ju, min(j0 + ku + p, n - 1));
+                named_sync(2, PT);
+                if (nz && p != jj) {
+                    if (tid < NB) {
+                        const double v = at(jj, tid);
+                        at(jj, tid) = at(p, tid);
+                        at(p, tid) = v;
+                    }
+                    pos = pos == jj ? p : (pos == p ? jj : pos);
+                }
+                if (tid == 0) {
+                    ip[j] = j0 + p;
+                    if (!nz) set_error(a.status, VERB_ERR_PIVOT);
+                }
+                named_sync(2, PT);
+                const double rcp = 1.0 / piv;
+#pragma unroll 1
+                for (int i = jj + 1 + tid; i <= jj + km; i += PT) {
+                    const double m = nz ? at(i, jj) * rcp : at(i, jj);
+                    Lf[(size_t)j * klp + (i - jj - 1)] = (T)m;
+                    at(i, jj) = nz ? m : 0.0;
+#pragma unroll 1
+                    for (int c = jj + 1; nz && c < NB; c++) {
+                        const double u = at(jj, c);
+                        if (u != 0.0) at(i, c) = fma(m, -u, at(i, c));
+                    }
+                }
+                named_sync(2, PT);
+            }
+        }
+        // the multipliers among the panel's rows, column by column from the
+        // diagonal down (negated, zero past row NB-1), for the triangular solves
+#pragma unroll
+        for (int e = tid; e < NB * NB; e += PT) {
+            const int m = e / NB, i = e % NB;
+            tri[(par * NB + m) * NB + i] = i && m + i < NB ? -W[off(m + i) + slot(m)] : 0.0;
+        }
+        // the interchanges as one permutation
+        if (pos < NB) s_src[par][pos] = off(t);
+        if (pos >= NB && pos != t) {
+            const int i = atomicAdd(&s_no[par], 1);
+            s_od[par][i] = off(pos);
+            s_os[par][i] = off(t);
+        }
+        if (tid == 0) {
+            s_ju[par] = ju;
+            s_bad[par] = bad;
+        }
+        return ju;
     };
-    fill_row(0, 0);
+
+    int ju0 = 0;  // the panel warps' running ju
+    // block j0: the panel at j0 is factored; j0 = -NB only factors the first
+    int rj = RW - NB, cj = CW - NB, par = 1;
+    for (int j0 = -NB;; j0 += NB, par ^= 1) {
+        const int jn = j0 + NB;  // next panel
+        const bool head = j0 < 0;
+        const int ju = head ? -1 : s_ju[par];
+        auto rslot = [&](int t) {
+            const int s = rj + t;
+            return (s >= RW ? s - RW : s) * pitch;
+        };
+        auto cslot = [&](int c) {  // column j0 + c
+            const int s = cj + c;
+            return s >= CW ? s - CW : s;
+        };
+        if (!head && wid == NW - 1) {
+            // U of the panel's own columns (and the padding below the diagonal)
+            const int k = lane % NB;
 #pragma unroll
-    for (int q = 0; q < NR; q++)
+            for (int i = 0; i < NB * NB / 32; i++) {
+                const int c = lane / NB + i * (32 / NB);
+                T* dst = Uf + (size_t)(j0 + c) * kvp + kv;
+                if (k <= c && j0 + c < n) dst[k - c] = (T)W[rslot(k) + cslot(c)];
+                if (k == c && j0 + c < n)
+                    for (int z = 1; z < kvp - kv; z++) dst[z] = (T)0;
+            }
+        }
+        if (jn >= n) break;
+        // Interchanges and the triangular solve of columns c < c_hi (relative to
+        // j0), one thread a column: U rows j0 .. jn-1 to the window.
+        auto solve_columns = [&](int c, int step, int c_hi, bool slow) {
+            const int no = s_no[par];
+            const double* tr = tri + par * NB * NB;
+#pragma unroll 1
+            for (; c < c_hi; c += step) {
+                double* col = W + cslot(c);
+                double x[NB];
 #pragma unroll
-        for (int k = 0; k < NC; k++) {
-            const int rs = wid + NW * q, cs = lane + 32 * k;
-            R[q][k] = (rs < RW && cs < CW && rs < n) ? row_value(rs, cs) : 0.0;
+                for (int k = 0; k < NB; k++) x[k] = col[s_src[par][k]];
+#pragma unroll 1
+                for (int i = 0; i < no; i += 4) {
+                    double y[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) y[e] = i + e < no ? col[s_os[par][i + e]] : 0.0;
+#pragma unroll
+                    for (int e = 0; e < 4; e++)
+                        if (i + e < no) col[s_od[par][i + e]] = y[e];
+                }
+                unsigned top = 0;
+                int r = rj;
+                // row m is always x[0]: the loop stays rolled; the next
+                // multipliers are loaded while these are used
+                double2 l[NB / 2];
+#pragma unroll
+                for (int k = 0; k < NB / 2; k++) l[k] = *(const double2*)(tr + 2 * k);
+#pragma unroll 1
+                for (int m = 0; m < NB; m++) {
+                    const double u = x[0];
+                    col[r * pitch] = u;
+                    r = r + 1 == RW ? 0 : r + 1;
+                    top = max(top, (unsigned)__double2hiint(u) & 0x7fffffffu);
+                    const double* tn = tr + min(m + 1, NB - 1) * NB;
+#pragma unroll
+                    for (int k = 0; k < NB / 2; k++) {
+                        const double2 lk = l[k];
+                        l[k] = *(const double2*)(tn + 2 * k);
+                        if (k) x[2 * k - 1] = slow && u == 0.0 ? x[2 * k] : fma(lk.x, u, x[2 * k]);
+                        x[2 * k] = slow && u == 0.0 ? x[2 * k + 1] : fma(lk.y, u, x[2 * k + 1]);
+                    }
+                }
+                if (top >= 0x7ff00000u) s_badu = 1;
+            }
+        };
+        // The update of columns c_lo .. c_hi-1 (relative to j0): warp w of nw
+        // takes 16 rows at a time, whose multipliers (negated) stay in
+        // registers, along all the columns, two 8-column tiles at a time.  With
+        // the row pitch at 2 or 14 mod 16 doubles, the tiles' row order (bits
+        // 0 and 1 of the index swapped) and columns (two pairs of a tile
+        // eight apart) keep the accesses to C and U free of bank conflicts.
+        auto update = [&](int c_lo, int c_hi, int w, int nw) {
+            const int g = lane >> 2, h = lane & 3;
+            const int gr = (g & 4) | (g & 1) << 1 | (g >> 1 & 1);
+            const int hc = 2 * (h >> 1) + 8 * (h & 1);           // of C
+            const int gc = 2 * (g >> 2) + 8 * (g >> 1 & 1) + (g & 1);  // of U
+            int rb[NB / 4];
+#pragma unroll
+            for (int k = 0; k < NB / 4; k++) rb[k] = rslot(4 * k + h);
+            for (int t0 = NB + 16 * w; t0 < RW; t0 += 16 * nw) {
+                int ro[2];
+                double l[2][NB / 4];
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    ro[i] = rslot(min(t0 + 8 * i + gr, RW - 1));
+#pragma unroll
+                    for (int k = 0; k < NB / 4; k++) l[i][k] = -W[ro[i] + cslot(4 * k + h)];
+                }
+                for (int c = c_lo; c < c_hi; c += 16) {
+                    double2 acc[2][2];
+                    int co[2];
+                    double u[2][NB / 4];
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        co[e] = cslot(min(c + 4 * e + hc, CW - 2));
+                        const int cb = cslot(min(c + 4 * e + gc, CW - 1));
+#pragma unroll
+                        for (int i = 0; i < 2; i++) acc[i][e] = *(const double2*)(W + ro[i] + co[e]);
+#pragma unroll
+                        for (int k = 0; k < NB / 4; k++) u[e][k] = W[rb[k] + cb];
+                    }
+#pragma unroll
+                    for (int k = 0; k < NB / 4; k++)
+#pragma unroll
+                        for (int e = 0; e < 2; e++)
+#pragma unroll
+                            for (int i = 0; i < 2; i++) dmma(acc[i][e], l[i][k], u[e][k]);
+#pragma unroll
+                    for (int e = 0; e < 2; e++)
+#pragma unroll
+                        for (int i = 0; i < 2; i++)
+                            if (t0 + 8 * i + gr < RW && c + 4 * e + hc < c_hi)
+                                *(double2*)(W + ro[i] + co[e]) = acc[i][e];
+                }
+            }
+        };
+        // the same update element by element with xGBTF2's skip (rows a pivot
+        // does not reach hold a zero multiplier)
+        auto update_slow = [&](int c_lo, int c_hi, int t, int nt) {
+            for (int e = t; e < (c_hi - c_lo) * kl; e += nt) {
+                const int c = c_lo + e / kl, r = NB + e % kl;
+                double v = W[rslot(r) + cslot(c)];
+                for (int k = 0; k < NB; k++) {
+                    const double u = W[rslot(k) + cslot(c)], l = W[rslot(r) + cslot(k)];
+                    if (u != 0.0 && l != 0.0) v = fma(l, -u, v);
+                }
+                W[rslot(r) + cslot(c)] = v;
+            }
+        };
+
+        // ---- the next panel's columns first
+        const bool slow_l = !head && s_bad[par] != 0;
+        const int cols_n = min(NB, n - jn);
+        if (!head) {
+        frw_wait_all();  // the entering rows
+        if (wid == 0) solve_columns(NB + lane, 32, NB + cols_n, slow_l);
+        __syncthreads();
+        // U rows j0 .. jn-1 of the next panel's columns out
+        for (int e = tid; e < NB * cols_n; e += NW * 32) {
+            const int k = e % NB, c = NB + e / NB;
+            if (c - k <= kv) Uf[(size_t)(j0 + c) * kvp + kv - (c - k)] = (T)W[rslot(k) + cslot(c)];
+        }
+        if (wid == NW - 1) {
+            // the entering rows' part in the next panel
+            for (int e = lane; e < NB * NB; e += 32) newp[e] = 0.0;
+            __syncwarp();
+            for (int e = lane; e < NB * 9; e += 32) {
+                const int r = e / 9, s = e - r * 9, q = j0 + RW + r;
+                const int c = q + diag_off(s) - jn;
+                if (q < n && c >= 0 && c < NB && jn + c < n)
+                    newp[r * NB + c] = stage[(par * NB + r) * 10 + s];
+            }
+        }
+        if (!(slow_l || s_badu)) {
+            update(NB, 2 * NB, wid, NW);
+        } else {
+            update_slow(NB, NB + cols_n, tid, NW * 32);
+        }
+        __syncthreads();
         }
 
-    int ju = 0;
-    int rj = 0, cj = 0;   // window slots of row j and column j (j mod RW, j mod CW)
-    for (int j = 0; j < n; j++) {
-        const int km = min(kl, n - 1 - j);
-        const int lc = cj & 31, kc = cj >> 5;
-        double* cv = colv + (j & 1) * RW;
-        // [top] this warp's candidate pivot in column j
-        if (lane == lc) {
-            // four interleaved first-maximum chains (rows q mod 4), merged at
-            // the end with the same rule: a shorter dependency chain than one
-            // pass over the thread's NR rows
-            double best[4] = {-1.0, -1.0, -1.0, -1.0};
-            int bi[4] = {1 << 30, 1 << 30, 1 << 30, 1 << 30};
-            frw_col(R, kc, [&](int q, double& val) {
-                const int rs = wid + NW * q;
-                int i = rs - rj;
-                if (i < 0) i += RW;
-                if (rs < RW && i <= km) {
-                    cv[i] = val;
-                    const double av = fabs(val);
-                    if (av > best[q & 3] || (av == best[q & 3] && i < bi[q & 3])) {
-                        best[q & 3] = av;
-                        bi[q & 3] = i;
-                    }
-                }
-            });
-#pragma unroll
-            for (int c = 1; c < 4; c++)
-                if (best[c] > best[0] || (best[c] == best[0] && bi[c] < bi[0])) {
-                    best[0] = best[c];
-                    bi[0] = bi[c];
-                }
-            s_best[wid] = best[0];
-            s_bi[wid] = bi[0];
-        }
-        __syncthreads();
-        // [B1] the pivot, the multipliers, the rows of the swap.  The NW
-        // candidates are combined by shuffles in every warp (lanes 0..NW-1
-        // hold them; the other lanes of each group carry empty candidates).
-        double best = lane < NW ? s_best[lane] : -1.0;
-        int jp = lane < NW ? s_bi[lane] : 1 << 30;
-        constexpr int GROUP = NW > 16 ? 32 : (NW > 8 ? 16 : 8);  // power of two >= NW
-#pragma unroll
-        for (int o = GROUP / 2; o > 0; o >>= 1) {
-            const double b = __shfl_xor_sync(0xffffffffu, best, o);
-            const int bi = __shfl_xor_sync(0xffffffffu, jp, o);
-            if (b > best || (b == best && bi < jp)) {
-                best = b;
-                jp = bi;
-            }
-        }
-        jp = __shfl_sync(0xffffffffu, jp, 0);
-        // idamax: a NaN first element is the maximum (nothing compares
-        // greater), elsewhere NaN never is
-        const double c0 = cv[0];
-        if (c0 != c0 || jp > km) jp = 0;
-        const double piv = cv[jp];
-        const bool nz = piv != 0.0;
-        const bool swap = nz && jp != 0;
-        const int rp = rj + jp < RW ? rj + jp : rj + jp - RW;
-        if (tid == 0) ip[j] = j + jp;
-        double rcp = 0.0;
-        if (nz) {
-            ju = max(ju, min(j + ku + jp, n - 1));
-            rcp = 1.0 / piv;
-            for (int i = 1 + tid; i <= km; i += blockDim.x) {
-                const double val = (i == jp) ? c0 : cv[i];
-                Lf[(size_t)j * klp + (i - 1)] = (T)(val * rcp);
-            }
+        int rjn = rj + NB, cjn = cj + NB;
+        if (rjn >= RW) rjn -= RW;
+        if (cjn >= CW) cjn -= CW;
+        if (wid < PW) {
+            ju0 = panel(jn, rjn, cjn, par ^ 1, head, ju0);
         } else {
-            if (tid == 0) set_error(a.status, VERB_ERR_PIVOT);
-            for (int i = 1 + tid; i <= km; i += blockDim.x) Lf[(size_t)j * klp + (i - 1)] = (T)cv[i];
-        }
-        {
-            // next column's entering row; its ring block must be present
-            const int qf = j + 1 + kl + 1;
-            if (j + 1 < n && qf < n && (qf & (STAGE_ROWS - 1)) == 0 && qf >= STAGE_ROWS) {
-                frw_wait_all();
-                __syncthreads();
-                if (qf + STAGE_ROWS < n) fetch_block(qf / STAGE_ROWS + 1);
+            // ---- the columns right of the next panel
+            const int ot = tid - PW * 32;
+            constexpr int ON = (NW - PW) * 32;
+            const int c_hi = ju - j0 + 1;   // columns c < c_hi take the update
+            solve_columns(2 * NB + ot, ON, c_hi, slow_l);
+            fetch_rows(jn, par ^ 1, ot, ON);
+            if (!head) {
+            named_sync(1, ON);
+            if (!(slow_l || s_badu)) {
+                update(2 * NB, min((c_hi + 1) & ~1, CW), wid - PW, NW - PW);
+            } else {
+                update_slow(2 * NB, c_hi, ot, ON);
             }
-            if (j + 1 < n) fill_row(j + 1, cj + 1 == CW ? 0 : cj + 1);
-        }
-        const bool own_j = wid == rj % NW;
-        const bool own_p = swap && wid == rp % NW;
-        const int qj = rj / NW, qp = rp / NW;
-        auto post = [&](double* dst) {
-            return [&, dst](double (&row)[NC]) {
+            // U rows j0 .. jn-1 out (lanes along the rows: contiguous in Uf)
+            {
+                const int k = ot % NB, c_end = min(min(NB + kv, n - j0), kv + k + 1);
+                const int rk = rslot(k);
+                T* dst = Uf + (size_t)j0 * kvp + kv + k;
+                constexpr int CS = ON / NB;
+                for (int c = 2 * NB + ot / NB; c < c_end; c += 4 * CS) {
+                    double v[4];
 #pragma unroll
-                for (int k = 0; k < NC; k++) {
-                    const int cs = lane + 32 * k;
-                    if (cs < CW) dst[cs] = row[k];
+                    for (int i = 0; i < 4; i++) v[i] = W[rk + cslot(min(c + i * CS, CW - 1))];
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        if (c + i * CS < c_end) dst[(size_t)(c + i * CS) * (kvp - 1)] = (T)v[i];
                 }
-            };
-        };
-        if (own_j) frw_row(R, qj, post(swap ? rowA : rowB));
-        if (own_p) frw_row(R, qp, post(rowB));
+            }
+            named_sync(1, ON);
+            // the slide: the panel's columns become columns j0 + CW .., its
+            // rows become the entering rows
+            const double2 z2 = make_double2(0.0, 0.0);
+#pragma unroll 4
+            for (int e = ot; e < (RW - NB) * (NB / 2); e += ON) {
+                const int r = e / (NB / 2), c = (e - r * (NB / 2)) * 2;
+                *(double2*)(W + rslot(NB + r) + cslot(c)) = z2;
+            }
+#pragma unroll 1
+            for (int c = 2 * ot; c < CW; c += 2 * ON)
+                if (c < NB || c >= 2 * NB) {
+                    double* col = W + cslot(c);
+#pragma unroll
+                    for (int r = 0; r < NB; r++) *(double2*)(col + rslot(r)) = z2;
+                }
+            named_sync(1, ON);
+            for (int e = ot; e < NB * 9; e += ON) {
+                const int r = e / 9, s = e - r * 9, q = j0 + RW + r;
+                const int c = q + diag_off(s) - j0;
+                if (q < n && c >= 2 * NB && j0 + c < n) {
+                    int cs = cj + c;
+                    while (cs >= CW) cs -= CW;
+                    W[rslot(r) + cs] = stage[(par * NB + r) * 10 + s];
+                }
+            }
+            }
+        }
         __syncthreads();
-        // [B2] swap, U row j, rank-1 update, slide
-        const int ncol = ju - j;   // columns j+1..ju take the update
-        int cofs[NC];              // column offset c - j of each owned slot
-#pragma unroll
-        for (int k = 0; k < NC; k++) {
-            int c = lane + 32 * k - cj;
-            if (c < 0) c += CW;
-            cofs[k] = c;
-        }
-        if (swap) {
-            auto take = [&](const double* src) {
-                return [&, src](double (&row)[NC]) {
-#pragma unroll
-                    for (int k = 0; k < NC; k++) {
-                        const int cs = lane + 32 * k;
-                        if (cs < CW && cofs[k] <= ncol) row[k] = src[cs];
-                    }
-                };
-            };
-            if (own_j) frw_row(R, qj, take(rowB));
-            if (own_p) frw_row(R, qp, take(rowA));
-        }
-        for (int c = j + tid; c <= ju && c <= j + kv; c += blockDim.x) {
-            const int cs = cj + (c - j) < CW ? cj + (c - j) : cj + (c - j) - CW;
-            Uf[(size_t)c * kvp + (kv - (c - j))] = (T)rowB[cs];
-        }
-        if (nz && km > 0 && ncol > 0) {
-            double ty[NC];
-#pragma unroll
-            for (int k = 0; k < NC; k++) {
-                const int cs = lane + 32 * k;
-                ty[k] = (cs < CW && cofs[k] >= 1 && cofs[k] <= ncol) ? -rowB[cs] : 0.0;
-            }
-#pragma unroll
-            for (int q = 0; q < NR; q++) {
-                const int rs = wid + NW * q;
-                int i = rs - rj;
-                if (i < 0) i += RW;
-                if (rs >= RW || i < 1 || i > km) continue;
-                const double m = ((i == jp) ? c0 : cv[i]) * rcp;
-                // xGER: A(i,k) + x(i)*temp with temp = -y(k), one fused
-                // multiply-add, skipped where temp = 0 (as a select, so that
-                // the lanes do not diverge)
-#pragma unroll
-                for (int k = 0; k < NC; k++) {
-                    const double u = fma(m, ty[k], R[q][k]);
-                    R[q][k] = ty[k] != 0.0 ? u : R[q][k];
-                }
-            }
-        }
-        // column slot cj now holds column j+CW, zero in every row but the new one
-        if (lane == lc) frw_col(R, kc, [](int, double& val) { val = 0.0; });
-        // row slot rj <- row j+kl+1 over columns j+1..j+CW (slot cs holds
-        // column j+1+((cs-(j+1)) mod CW))
-        if (own_j)
-            frw_row(R, qj, [&](double (&row)[NC]) {
-#pragma unroll
-                for (int k = 0; k < NC; k++) {
-                    const int cs = lane + 32 * k;
-                    row[k] = cs < CW ? nrow[(j & 1) * CW + cs] : 0.0;
-                }
-            });
-        if (++rj == RW) rj = 0;
-        if (++cj == CW) cj = 0;
+        rj = rjn;
+        cj = cjn;
     }
 }
 
@@ -1741,54 +2002,50 @@ size_t local_factor_smem(int V)
 
 namespace {
 
-template <typename T, int NR, int NC, int NW>
-void launch_factor_rw(const LocalArgs& a, cudaStream_t s)
+template <typename T, int PW, int NW>
+void launch_factor_blk(const LocalArgs& a, cudaStream_t s)
 {
     const int kl = a.d.V + 1, kv = 2 * kl;
     dim3 g((a.d.V * a.d.K + 255) / 256, a.d.P * a.d.R);
     local_rows_kernel<T><<<g, 256, 0, s>>>(a);
-    const size_t smem = ((size_t)2 * STAGE_ROWS * 9 + 4 * (kv + 1) + 2 * (kl + 1)) * sizeof(double);
-    allow_max_dynamic_smem((const void*)local_factor_rw_kernel<T, NR, NC, NW>);
-    local_factor_rw_kernel<T, NR, NC, NW><<<a.d.P * a.d.R, NW * 32, smem, s>>>(a);
+    FBlk f{kl + NB, kv + NB, kv + NB};
+    while (f.pitch % 16 != 2 && f.pitch % 16 != 14) f.pitch += 2;
+    const size_t smem = ((size_t)f.RW * f.pitch + 2 * NB * 10 + NB * NB + 2 * PW * (NB + 4) + 2 * NB * NB) * sizeof(double);
+    allow_max_dynamic_smem((const void*)local_factor_blk_kernel<T, PW, NW>);
+    local_factor_blk_kernel<T, PW, NW><<<a.d.P * a.d.R, NW * 32, smem, s>>>(a, f);
 }
 
-// Eight warps hold the register window.  Twelve and sixteen warps (fewer
-// slots and instructions per thread) were measured no faster at V = 101
-// (1.20 s and 1.42 s against 1.19 s for 48 x 101 x 101 x 91): the column
-// chain, not the per-thread work, sets the time.
-constexpr int FRW_WARPS = 8;
-
-// Register window shape: NC = ceil((kv+1)/32) column slots per lane and
-// NR = ceil((kl+1)/8) row slots per thread, NR in {2 NC - 1, 2 NC} since
-// kv + 1 = 2 (kl+1) - 1.  NC <= 7 keeps the window in 255 registers
-// (V <= 110); wider bands take local_factor_kernel.
 template <typename T>
-bool launch_factor_rw_t(const LocalArgs& a, cudaStream_t s)
+bool launch_factor_blk_t(const LocalArgs& a, cudaStream_t s)
 {
-    const int RW = a.d.V + 2, CW = 2 * (a.d.V + 1) + 1;
-    const int nc = (CW + 31) / 32, nr = (RW + FRW_WARPS - 1) / FRW_WARPS;
-    if (nc > 7 || (nr != 2 * nc && nr != 2 * nc - 1)) return false;
     // a parked row needs 9 doubles of an L column; systems index grid.y of
     // the parking launch
     if (a.factors32 ? a.klp32 < 18 : a.klp < 9) return false;
     if (a.d.P * a.d.R > 65535) return false;
-#define VERB_FRW(NR, NC)                                                              \
-    if (nc == NC && nr == NR) {                                                       \
-        launch_factor_rw<T, NR, NC, FRW_WARPS>(a, s);                                 \
-        return true;                                                                  \
-    }
-    VERB_FRW(1, 1) VERB_FRW(2, 1) VERB_FRW(3, 2) VERB_FRW(4, 2) VERB_FRW(5, 3) VERB_FRW(6, 3)
-    VERB_FRW(7, 4) VERB_FRW(8, 4) VERB_FRW(9, 5) VERB_FRW(10, 5) VERB_FRW(11, 6) VERB_FRW(12, 6)
-    VERB_FRW(13, 7) VERB_FRW(14, 7)
-#undef VERB_FRW
-    return false;
+    // PW: the kl + NB rows of a panel, one a thread.  Measured (GPU time of an
+    // upload-factorise-solve pass): 24 x 51 x 101 x 21 with 4 + 8 warps 18.9 ms
+    // (4 + 12: 19.3, 4 + 4: 22.9; panels of 16 columns 19.5-21.5);
+    // 24 x 25 x 31 x 31 with 2 + 2 warps 3.6 ms alone (2 + 4: 4.0; 16 columns 4.2).
+    const int kl = a.d.V + 1;
+    if (kl + NB <= 32) launch_factor_blk<T, 1, 3>(a, s);
+    else if (kl + NB <= 64) launch_factor_blk<T, 2, 4>(a, s);
+    else if (kl + NB <= 96) launch_factor_blk<T, 3, 9>(a, s);
+    else launch_factor_blk<T, 4, 12>(a, s);
+    return true;
 }
 
 }  // namespace
 
 int launch_local_factor(const LocalArgs& a, cudaStream_t s)
 {
-    if (a.factors32 ? launch_factor_rw_t<float>(a, s) : launch_factor_rw_t<double>(a, s)) return 2;
+    // The blocked kernel writes every entry of Uf (above row 0 and the padding
+    // included) of the systems it factors; where some are skipped, and for the
+    // window kernel, Uf is cleared first.
+    const bool blk = a.factors32 ? a.klp32 >= 18 : a.klp >= 9;
+    if (!(blk && a.d.P * a.d.R <= 65535) || !a.include_boundary || a.k0 || a.sel)
+        cudaMemsetAsync(a.factors32 ? (void*)a.Uf32 : (void*)a.Uf, 0,
+                        a.unknowns * (a.factors32 ? a.kvp32 * sizeof(float) : a.kvp * sizeof(double)), s);
+    if (a.factors32 ? launch_factor_blk_t<float>(a, s) : launch_factor_blk_t<double>(a, s)) return 2;
     const size_t smem = local_factor_smem(a.d.V);
     if (a.factors32) {
         allow_max_dynamic_smem((const void*)local_factor_kernel<float>);

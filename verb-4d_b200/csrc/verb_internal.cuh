@@ -149,6 +149,7 @@ struct LocalArgs {
     // != 0 are processed
     const unsigned char* sel;
     unsigned char sel_mask;
+    size_t unknowns;    // of all systems
     int32_t* ipiv;      // [sys][n]        0-based pivot rows
     double* work;       // [sys][n]        rhs / solution in unknown order (iK*V + iV)
     unsigned long long* negatives;  // optional: count of PSD < 0 written by the store kernel
