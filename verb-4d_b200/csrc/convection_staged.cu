@@ -1,0 +1,642 @@
+// Convection in (MLT, L) on every (V,K) slice, a QUICKEST pass in two stages
+// over line segments: Convection_2D (src/Convection_2D.cpp:36-169) over
+// Convection_1D_ULTIMATE_QUICKEST6 (QUICKEST6.cpp:22-482), contracted like
+// convection_stream.cu, whose face polynomial, limiter and tables it shares.
+//
+// A CTA keeps one [P][R] slice in shared memory for all of its CFL sub-steps.
+// The reference's four loops over a line become two, each run by one thread
+// per segment of a line (about 4 to 13 cells, threads of a warp on
+// neighbouring lines):
+//   stage 1  unlimited faces a .. a+own and from them the unlimited cells
+//            (loops 1 and 2, :148-272), both to shared memory;
+//   stage 2  the peak flags of the segment as bit masks from the unlimited
+//            line, then limited faces and final cells (loops 3 and 4,
+//            :277-477), in place, with the store epilogue.
+// A barrier separates the stages and the sweeps.  The face between two
+// segments is formed by both; what a segment reads of its neighbours' cells in
+// stage 2, it keeps in registers from stage 1.
+//
+// What bounds it: the issue of about 240 instructions a face (a third of them
+// FP64), with 16 warps on an SM.  The streaming kernel (one thread a line, all
+// four loops at once) holds some 40 values in flight, which limits it to 12
+// warps whose chains run along the whole line, so a slice of many sub-steps
+// takes as long as its lines are: 24 x 25 x 31 x 31 alone 9.9 ms, 3.4 here
+// (three runs at once 3.78 -> 1.18 ms each); 48 x 101 x 101 x 16 alone 47.4 ms,
+// 23.2 here (one after the other 31.0 -> 23.1 ms).  What the groups and layouts
+// below measured at the latter size is said beside them.
+#include "conv_stream.cuh"
+#include "verb_internal.cuh"
+
+#include <algorithm>
+
+namespace verb {
+namespace {
+
+constexpr double CG_MAX_SUBSTEPS = 1.0e6;
+constexpr int CG_MAX_OWN = 25;  // cells of a segment: own + 7 flag bits in a word
+
+// The planes carry CG_GH ghost cells around the slice, so that a window never
+// needs to ask where the line ends.
+constexpr int CG_GH = 5;
+__host__ __device__ inline int cg_rs(int R) { return (R + 2 * CG_GH) | 1; }
+
+// Launch shape of a [P][R] slice.
+struct StagedShape {
+    int threads;      // per CTA
+    int segP, segR;   // segments of an MLT line, of an L line
+};
+
+// per CTA: c and 1/|c| of both sweeps' faces, the store epilogues (factor, and
+// added term of the L sweep), line data, and room for the rows a group reads
+// past a line's end
+__host__ __device__ inline size_t cg_scratch(int P, int R)
+{
+    return 2 * (size_t)P * (R - 1) + 5 * (size_t)P * R + 4 * (size_t)(R - 1) + 4 * (size_t)P +
+           32 * (size_t)(P > R ? P : R);
+}
+
+__host__ __device__ inline size_t cg_plane(int P, int R)
+{
+    return (size_t)(P + 2 * CG_GH) * cg_rs(R);
+}
+
+// three planes and what a group reads past the last one
+__host__ __device__ inline size_t cg_smem(int P, int R)
+{
+    return (3 * cg_plane(P, R) + 8 * (size_t)cg_rs(R) + 32) * sizeof(double) +
+           (size_t)(R + P) * sizeof(int);
+}
+
+// A thread's segment of a line.
+struct Seg {
+    const double* E;     // cell k of the line before the pass at [k * st], with ghosts
+    double* U;           // unlimited cell k, with ghosts
+    double* O;           // unlimited face k + 1, replaced by cell k after the pass
+    int st;
+    int a, own, n;       // first cell, cells, points of the line
+    int lt, ut;
+    const double* ln;    // line data (lbc, ubc, dxl, dxu) at ln[i * nl]
+    int nl;
+    const double *cr, *rc;  // c and 1 / |c| (0 for |c| <= 1e-31) of face k at [k * nl]
+    const double *e1, *e2;  // store epilogue of cell k: times e1, plus e2 (or nullptr)
+};
+
+// ghost cells of the line before a pass (:89-143)
+__device__ __forceinline__ void line_ghosts(double* E, int st, int n, int lt, int ut,
+                                            const double* ln, int nl)
+{
+    if (lt == VERB_BC_PERIODIC) {
+#pragma unroll
+        for (int k = 1; k <= CG_GH; k++) {
+            E[-k * st] = E[(n - 1 - k) * st];
+            E[(n - 1 + k) * st] = E[k * st];
+        }
+        return;
+    }
+    double g = E[0], h = E[(n - 1) * st];
+    const double dl = ln[0] * ln[2 * nl], du = ln[nl] * ln[3 * nl];
+#pragma unroll
+    for (int k = 1; k <= CG_GH; k++) {
+        g = lt == VERB_BC_CONSTANT_VALUE ? ln[0] : g - dl;
+        h = ut == VERB_BC_CONSTANT_VALUE ? ln[nl] : h + du;
+        E[-k * st] = g;
+        E[(n - 1 + k) * st] = h;
+    }
+}
+
+// Stage 1 takes the faces of a segment CG_U at a time, stage 2 CG_W: the
+// polynomials and the limiters of a group are independent of each other, and
+// the window is loaded once per group instead of shifted through registers.
+// Groups of 6 and 3: 23.2 ms (4 and 4: 28.8, spilling; 12 and 4: 34.0; 6 and 6:
+// 24.3; a window shifted face by face 29.8).
+constexpr int CG_U = 6, CG_W = 3;
+
+// Unlimited values of U faces from the window d[k] = E[x-5+k] (QUICKEST6.cpp:
+// 162-241, in the positive orientation with the signed Courant number).  The
+// differences of the stencil are built level by level for all of the group's
+// faces, D^m_k = D^(m-1)_k - D^(m-1)_(k+1), shared by neighbouring faces: with
+// (a, b) the two m-th differences at face u, m even, the reference's even term
+// is (a + b) / 2 and its odd term a - b.  The ninth-order pair E8 + sign d9 is
+// 2a or 2b.
+template <int U>
+__device__ __forceinline__ void faces(double (&d)[U + 9], const double (&c)[U], double (&f)[U])
+{
+    double cs[U], p[U];
+    auto level = [&](int m) {  // next difference, in place: m entries
+#pragma unroll
+        for (int k = 0; k < U + 8; k++)
+            if (k < m) d[k] = d[k] - d[k + 1];
+    };
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const double s0 = d[u + 4] + d[u + 5];
+        const double t0 = d[u + 4] - d[u + 5];
+        f[u] = 0.5 * (s0 + c[u] * t0);
+        cs[u] = c[u] * c[u];
+        p[u] = cs[u] - 1;
+    }
+    level(U + 8);
+    level(U + 7);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const double x = d[u + 3], y = d[u + 4];
+        f[u] += (p[u] * (1.0 / 12.0)) * ((x + y) + (c[u] * 0.5) * (x - y));
+        p[u] *= cs[u] - 4;
+    }
+    level(U + 6);
+    level(U + 5);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const double x = d[u + 2], y = d[u + 3];
+        f[u] += (p[u] * (1.0 / 240.0)) * ((x + y) + (c[u] * (1.0 / 3.0)) * (x - y));
+        p[u] *= cs[u] - 9;
+    }
+    level(U + 4);
+    level(U + 3);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const double x = d[u + 1], y = d[u + 2];
+        f[u] += (p[u] * (1.0 / 10080.0)) * ((x + y) + (c[u] * 0.25) * (x - y));
+        p[u] *= cs[u] - 16;
+    }
+    level(U + 2);
+    level(U + 1);
+#pragma unroll
+    for (int u = 0; u < U; u++)
+        f[u] += (p[u] * (1.0 / 362880.0)) * (c[u] >= 0 ? d[u] : d[u + 1]);
+}
+
+// returns unlimited face a, whose slot is the neighbour's
+__device__ __forceinline__ double stage1(const Seg& L)
+{
+    constexpr int U = CG_U;
+    double Q = 0.0, f0 = 0.0;
+    const double* cp = L.cr + L.a * L.nl;
+    // faces a .. a+own, cells a .. a+own-1; what is read past the line's
+    // ghosts and tables (memory of the same regions) only feeds faces past own
+#pragma unroll 1
+    for (int i = 0; i <= L.own; i += U) {
+        const int x = L.a + i;
+        double d[U + 9], c[U], f[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) c[u] = cp[u * L.nl];
+        cp += U * L.nl;
+        const double* ep = L.E + (x - 5) * L.st;
+#pragma unroll
+        for (int k = 0; k < U + 9; k++) d[k] = ep[k * L.st];
+        faces<U>(d, c, f);
+        double* up = L.U + (x - 1) * L.st;
+        double* fp = L.O + (x - 1) * L.st;
+        if (i == 0) f0 = f[0];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const double q = c[u] * f[u];
+            if ((u > 0 || i > 0) && i + u <= L.own) {
+                up[u * L.st] = ep[(u + 4) * L.st] - (q - Q);
+                fp[u * L.st] = f[u];
+            }
+            Q = q;
+        }
+    }
+    const double* ep = L.E + L.a * L.st;
+    // boundary rewrite (:257-272) and the unlimited line's ghosts (:281-330;
+    // the periodic low ones come from the line before the pass)
+    if (L.lt == VERB_BC_PERIODIC) {
+        if (L.a == 0) {
+            L.U[(L.n - 1) * L.st] = L.U[0];
+#pragma unroll
+            for (int k = 1; k <= 4; k++) L.U[-k * L.st] = ep[-k * L.st];
+        }
+        if (L.a <= 4)
+            for (int k = max(1, L.a); k <= min(4, L.a + L.own - 1); k++)
+                L.U[(L.n - 1 + k) * L.st] = L.U[k * L.st];
+        return f0;
+    }
+    if (L.a == 0) {
+        const double u0 = L.lt == VERB_BC_CONSTANT_VALUE ? L.ln[0] : L.U[L.st];
+        const double dl = L.ln[0] * L.ln[2 * L.nl];
+        double g = u0;
+        L.U[0] = u0;
+#pragma unroll
+        for (int k = 1; k <= 4; k++) {
+            g = L.lt == VERB_BC_CONSTANT_VALUE ? u0 : g - dl;
+            L.U[-k * L.st] = g;
+        }
+    }
+    if (L.a + L.own == L.n - 1) {
+        double* e = L.U + (L.n - 1) * L.st;
+        const double u1 = L.ut == VERB_BC_CONSTANT_VALUE ? L.ln[L.nl] : e[-L.st];
+        const double du = L.ln[L.nl] * L.ln[3 * L.nl];
+        double g = u1;
+        e[0] = u1;
+#pragma unroll
+        for (int k = 1; k <= 4; k++) {
+            g = L.ut == VERB_BC_CONSTANT_VALUE ? u1 : g + du;
+            e[k * L.st] = g;
+        }
+    }
+    return f0;
+}
+
+// v with its sign flipped where s is the sign bit
+__device__ __forceinline__ double flip(double v, int s)
+{
+    return __hiloint2double(__double2hiint(v) ^ s, __double2loint(v));
+}
+
+// Limited face value (:394-447) from the unlimited value f, the Courant
+// number c and 1 / |c|, cells x-2 .. x+1 and the face's peak flag.
+__device__ __forceinline__ double limit(double f, double c, double rc, double em2, double em1,
+                                        double e0, double ep1, bool peak)
+{
+    const bool pos = c >= 0;
+    const double ou = pos ? em2 : ep1;
+    const double oc = pos ? em1 : e0;
+    const double od = pos ? e0 : em1;
+    const double DEL = od - ou;
+    const double CURV = od - 2 * oc + ou;
+    // not flat implies DEL != 0 (where it is NaN, so is f and what follows)
+    const bool flat = fabs(CURV) >= fabs(DEL);
+    const bool useref = !peak & !flat & (__double2hiint(rc) != 0);
+    const double ref = ou + (oc - ou) * rc;
+    const int s = DEL > 0 ? 0 : (int)0x80000000;
+    const double a = flip(f, s), lo = flip(oc, s), h1 = flip(ref, s), h2 = flip(od, s);
+    double t = a > lo ? a : lo;
+    const double hi = h1 < h2 ? h1 : h2;
+    t = t < hi ? t : hi;
+    double res = useref ? flip(t, s) : f;
+    if (!peak & flat) res = oc;
+    return res;
+}
+
+// last: the line's last sub-cycle, whose cells take the store epilogue
+__device__ __forceinline__ void stage2(const Seg& L, double f0, bool last)
+{
+    // peak flags M of positions a-4 .. : differences e_k = U[k+1] - U[k], bit
+    // k - (a-4); M: rising twice, then falling twice, with a bend at both ends
+    unsigned up = 0, dn = 0, bend = 0;
+    {
+        constexpr int W = 6;
+        const double* p = L.U + (L.a - 4) * L.st;
+        double v = *p, e = 0.0;
+#pragma unroll 1
+        for (int i = 0; i < L.own + 7; i += W) {
+            double w[W];
+#pragma unroll
+            for (int u = 0; u < W; u++) {
+                p += L.st;
+                w[u] = *p;
+            }
+            unsigned b1 = 0, b2 = 0, b3 = 0;
+#pragma unroll
+            for (int u = 0; u < W; u++) {
+                const double en = w[u] - v;
+                if (en > 0) b1 |= 1u << u;
+                if (en < 0) b2 |= 1u << u;
+                if (en < e) b3 |= 1u << u;
+                v = w[u];
+                e = en;
+            }
+            up |= b1 << i;
+            dn |= b2 << i;
+            bend |= b3 << i;
+        }
+        bend >>= 1;
+    }
+    const unsigned M = up & up >> 1 & dn >> 2 & dn >> 3 & bend & bend >> 2;
+    // face x takes positions x-4 .. x-2, or x-3 .. x-1 against the direction
+    unsigned three = M | M >> 1 | M >> 2;
+
+    constexpr int U = CG_W;
+    double Rp = 0.0, first = 0.0, second = 0.0, end = 0.0;
+    int at = L.a * L.nl;
+#pragma unroll 1
+    for (int i = 0; i <= L.own; i += U) {
+        const int x = L.a + i;
+        const double* ep = L.E + (x - 2) * L.st;
+        double* op = L.O + (x - 1) * L.st;
+        double c[U], rc[U], h1[U], h2[U], w[U + 3], f[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            c[u] = L.cr[at];
+            rc[u] = L.rc[at];
+            h1[u] = 1.0;
+            h2[u] = 0.0;
+            at += L.nl;
+            // cell x + u - 1 (the first group's entry of cell a - 1, and past
+            // the table's ends, is not used)
+            if (last) {
+                h1[u] = L.e1[at - 2 * L.nl];
+                if (L.e2) h2[u] = L.e2[at - 2 * L.nl];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < U + 3; k++) w[k] = ep[k * L.st];
+#pragma unroll
+        for (int u = 0; u < U; u++) f[u] = op[u * L.st];
+        if (i == 0) f[0] = f0;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const bool peak = three >> (u + (c[u] >= 0 ? 0 : 1)) & 1u;
+            const double r = c[u] * limit(f[u], c[u], rc[u], w[u], w[u + 1], w[u + 2], w[u + 3],
+                                          peak);
+            const double o = w[u + 1] - (r - Rp);
+            if ((u > 0 || i > 0) && i + u <= L.own) op[u * L.st] = o * h1[u] + h2[u];
+            if (u == 1 && i == 0) first = o;
+            if (u == 2 && i == 0) second = o;
+            if (L.ut == VERB_BC_CONSTANT_DERIVATIVE && i + u == L.own) end = o;
+            Rp = r;
+        }
+        three >>= U;
+    }
+    // boundary rewrite (:462-477): the cells at the line's ends (no source term)
+    auto put = [&](int k, double v) { L.O[k * L.st] = last ? v * L.e1[k * L.nl] : v; };
+    if (L.a == 0) {
+        if (L.lt == VERB_BC_PERIODIC) put(L.n - 1, first);
+        else put(0, L.lt == VERB_BC_CONSTANT_VALUE ? L.ln[0] : second);
+    }
+    if (L.a + L.own == L.n - 1 && L.ut != VERB_BC_PERIODIC)
+        put(L.n - 1, L.ut == VERB_BC_CONSTANT_VALUE ? L.ln[L.nl] : end);
+}
+
+__device__ __forceinline__ double cg_block_max(double v, double* red)
+{
+    for (int o = 16; o > 0; o >>= 1) {
+        const double t = __shfl_xor_sync(0xffffffffu, v, o);
+        v = (v < t) ? t : v;
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    __syncthreads();
+    if (lane == 0) red[warp] = v;
+    __syncthreads();
+    double m = red[0];
+    for (int i = 1; i < nw; i++) m = (m < red[i]) ? red[i] : m;
+    __syncthreads();
+    return m;
+}
+
+template <int MAXT, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs a, int segP, int segR)
+{
+    extern __shared__ __align__(16) double sm[];
+    const Dims d = a.d;
+    const int P = d.P, R = d.R, V = d.V, K = d.K;
+    const int PR = P * R, Rs = cg_rs(R);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nt = blockDim.x, nw = nt >> 5;
+    const int plane = (int)cg_plane(P, R);
+    double* S = sm + CG_GH * Rs + CG_GH;    // the slice, with ghosts
+    double* F = S + plane;                  // unlimited faces, then the slice after a sweep
+    double* U = F + plane;                  // unlimited cells of a sweep, with ghosts
+    double* red = sm + 3 * (size_t)plane + 8 * (size_t)Rs;  // [32]
+    int* nsP = (int*)(red + 32);            // [R] sub-cycles of P-line iR
+    int* nsR = nsP + R;                     // [P] sub-cycles of R-line iP
+    __shared__ int s_ticket, s_ns[2];
+
+    // slice tables, line-fastest: [P faces or cells][R-1 lines], [R][P lines]
+    const size_t VK = (size_t)V * K, P1 = (size_t)P * (R - 1);
+    double* crP = a.scratch + (size_t)blockIdx.x * cg_scratch(P, R);
+    double* rcP = crP + P1;
+    double* e1P = rcP + P1;                    // G
+    double* crR = e1P + (size_t)PR;
+    double* rcR = crR + (size_t)PR;
+    double* e1R = rcR + (size_t)PR;            // exp(Loss dt)/G
+    double* e2R = e1R + (size_t)PR;            // S dt, 0 at the ends
+    double* lnP = e2R + (size_t)PR;            // [4][R-1]
+    double* lnR = lnP + 4 * (size_t)(R - 1);   // [4][P]
+    const int nslices = V * K;
+
+    for (;;) {
+        if (tid == 0) {
+            s_ticket = atomicAdd(a.ticket, 1);
+            s_ns[0] = s_ns[1] = 1;
+        }
+        __syncthreads();
+        const int t = s_ticket;
+        __syncthreads();
+        if (t >= nslices) break;
+        const int iV = V - 1 - t / K;
+        const int iK = t - (t / K) * K;
+        const size_t off = (size_t)iV * K + iK;
+        auto g = [&](int iP, int iR) { return ((size_t)iP * R + iR) * VK + off; };
+
+        // slice load and slice-level sub-step count (src/Convection_2D.cpp:57-86)
+        double vpm = 0.0, vrm = 0.0;
+        for (int i = tid; i < PR; i += nt) {
+            const int iP = i / R, iR = i - iP * R;
+            const size_t gi = g(iP, iR);
+            S[iP * Rs + iR] = a.psd[gi];
+            const double vp = fabs(a.VP[gi]), vr = fabs(a.VR[gi]);
+            vpm = (vpm < vp) ? vp : vpm;
+            vrm = (vrm < vr) ? vr : vrm;
+        }
+        vpm = cg_block_max(vpm, red);
+        vrm = cg_block_max(vrm, red);
+        double nsp, nsr;
+        {
+            const double dP = a.Pg[g(1, 0)] - a.Pg[g(0, 0)];
+            const double x = (double)a.dt * vpm / dP / 0.25;
+            nsp = x <= 1 ? 1 : ceil(x);
+        }
+        {
+            const double dR = a.Rg[g(0, 1)] - a.Rg[g(0, 0)];
+            const double x = (double)a.dt * vrm / dR / 0.25;
+            nsr = x <= 1 ? 1 : ceil(x);
+        }
+        const double num_steps = (nsp < nsr) ? nsr : nsp;
+        if (!(num_steps <= CG_MAX_SUBSTEPS)) {  // also catches inf / NaN
+            if (tid == 0) {
+                a.substeps[off] = -1;
+                set_error(a.status, VERB_ERR_CFL);
+            }
+            __syncthreads();
+            continue;
+        }
+        const double dtc = a.dt / num_steps;
+        if (tid == 0) a.substeps[off] = (int)num_steps;
+        for (int i = tid; i < PR; i += nt) {
+            const int iP = i / R, iR = i - iP * R;
+            const size_t gi = g(iP, iR);
+            const double G = a.G[gi];
+            if (iR < R - 1) e1P[(size_t)iP * (R - 1) + iR] = G;
+            e1R[(size_t)iR * P + iP] = exp(a.loss[gi] * dtc) / G;
+            e2R[(size_t)iR * P + iP] = iR && iR < R - 1 ? a.S[gi] * dtc : 0.0;
+        }
+        // per-line CFL sub-cycles and face Courant numbers (QUICKEST6.cpp:37-52,
+        // 150-160), one warp per line; velocity vel and grid x at (line, k)
+        auto line_table = [&](const double* vel, const double* x, int line, int n, bool pr,
+                              double* cr, double* rc, int* nsl, double* ln, int nl) {
+            auto at = [&](int k) { return pr ? g(k, line) : g(line, k); };
+            double m = -INFINITY;
+            for (int k = lane; k < n; k += 32) {
+                const double v = fabs(vel[at(k)]);
+                m = (m > v) ? m : v;
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                const double q = __shfl_xor_sync(0xffffffffu, m, o);
+                m = (m > q) ? m : q;
+            }
+            const double dx = x[at(1)] - x[at(0)];
+            const double sd = (double)dtc * m / dx / 1.0;
+            int ns = 1;
+            if (!(sd <= CG_MAX_SUBSTEPS)) set_error(a.status, VERB_ERR_CFL);
+            else if (sd > 1) ns = (int)ceil(sd);
+            const double dtl = dtc / ns;
+            if (fabs(m / dx * dtl) > 1) set_error(a.status, VERB_ERR_CFL);
+            for (int k = lane; k < n; k += 32) {
+                const double c0 = vel[at(k == 0 ? n - 2 : k - 1)] / dx * dtl;
+                const double c1 = vel[at(k)] / dx * dtl;
+                const double c = (c0 + c1) / 2;
+                cr[(size_t)k * nl + line] = c;
+                rc[(size_t)k * nl + line] = fabs(c) > 1e-31 ? __drcp_rn(fabs(c)) : 0.0;
+            }
+            if (lane == 0) {
+                nsl[line] = ns;
+                if (ns > 1) atomicMax(&s_ns[pr ? 0 : 1], ns);
+                ln[2 * nl + line] = dx;
+                ln[3 * nl + line] = x[at(n - 1)] - x[at(n - 2)];
+            }
+        };
+        for (int iR = warp; iR < R - 1; iR += nw) {
+            line_table(a.VP, a.Pg, iR, P, true, crP, rcP, nsP, lnP, R - 1);
+            if (lane == 0) {
+                const size_t bo = ((size_t)iR * V + iV) * K + iK;
+                lnP[iR] = a.Pl[bo];
+                lnP[(R - 1) + iR] = a.Pu[bo];
+            }
+        }
+        for (int iP = warp; iP < P; iP += nw) {
+            line_table(a.VR, a.Rg, iP, R, false, crR, rcR, nsR, lnR, P);
+            if (lane == 0) {
+                const size_t bo = ((size_t)iP * V + iV) * K + iK;
+                lnR[iP] = a.Rl[bo] * a.G[g(iP, 0)];
+                lnR[P + iP] = a.Ru[bo] * a.G[g(iP, R - 1)];
+            }
+        }
+        __syncthreads();
+
+        for (int it = 0; it < num_steps; it++) {
+            // the MLT sweep (ph 0: P-lines iR, stored times G) and the L sweep
+            // (ph 1: R-lines iP, stored as v exp(Loss dt)/G + S dt) go through
+            // one copy of the stages
+#pragma unroll 1
+            for (int ph = 0; ph < 2; ph++) {
+                const bool pr = ph == 0;
+                const int nl = pr ? R - 1 : P, ns_seg = pr ? segP : segR;
+                const int seg = tid / nl, line = tid - seg * nl;
+                Seg L;
+                L.n = pr ? P : R;
+                // the n-1 cells before the last, in segments of two lengths
+                const int nc = L.n - 1, len = nc / ns_seg, more = nc - len * ns_seg;
+                L.own = len + (seg < more);
+                L.a = seg * len + min(seg, more);
+                const bool live = seg < ns_seg;
+                L.st = pr ? Rs : 1;
+                const int o0 = pr ? line : line * Rs;
+                L.U = U + o0;
+                L.lt = pr ? a.Pl_t : a.Rl_t;
+                L.ut = pr ? a.Pu_t : a.Ru_t;
+                L.ln = (pr ? lnP : lnR) + line;
+                L.nl = nl;
+                L.cr = (pr ? crP : crR) + line;
+                L.rc = (pr ? rcP : rcR) + line;
+                L.e1 = (pr ? e1P : e1R) + line;
+                L.e2 = pr ? nullptr : e2R + line;
+                const int ns = live ? (pr ? nsP : nsR)[line] : 0;
+                // the line's own CFL sub-cycles (:37-52), the epilogue on the
+                // last one only
+                const int most = s_ns[ph];
+                for (int k = 0; k < most; k++) {
+                    for (int q = tid; q < nl; q += nt) {
+                        double* e = S + (pr ? q : q * Rs);
+                        line_ghosts(e, L.st, L.n, L.lt, L.ut, (pr ? lnP : lnR) + q, nl);
+                    }
+                    L.E = S + o0;
+                    L.O = F + o0;
+                    const bool run = k < ns, last = k == ns - 1;
+                    double f0 = 0.0;
+                    __syncthreads();
+                    if (run) f0 = stage1(L);
+                    __syncthreads();
+                    if (run) {
+                        stage2(L, f0, last);
+                    } else if (live) {  // this line is done: carried over
+                        for (int x = L.a; x < L.a + L.own + (seg == ns_seg - 1); x++)
+                            L.O[x * L.st] = L.E[x * L.st];
+                    }
+                    // the last L row, which the MLT sweep does not touch (:104)
+                    if (pr)
+                        for (int iP = nt - 1 - tid; iP < P; iP += nt) {
+                            const double v = S[iP * Rs + R - 1];
+                            F[iP * Rs + R - 1] = k == 0 ? v * a.G[g(iP, R - 1)] : v;
+                        }
+                    __syncthreads();
+                    double* t2 = S;
+                    S = F;
+                    F = t2;
+                }
+            }
+        }
+        for (int i = tid; i < PR; i += nt) {
+            const int iP = i / R, iR = i - iP * R;
+            a.psd[g(iP, iR)] = S[iP * Rs + iR];
+        }
+        __syncthreads();
+    }
+}
+
+constexpr int CG_MAXT = 512;  // 125 registers a thread
+constexpr int CG_MINB = 1;
+
+// Segments whose faces fill whole groups: of 5 cells on small slices, where a
+// sub-step's chain is what a pass waits for, of 11 on others, longer where the
+// lines would need more threads than a CTA has.
+bool cg_shape(int P, int R, StagedShape& s)
+{
+    for (int own = P * R < 1200 ? CG_U - 1 : 2 * CG_U - 1; own <= CG_MAX_OWN; own += CG_U) {
+        s.segP = std::max(1, std::min((P - 1 + own - 1) / own, (P - 1) / 4));
+        s.segR = std::max(1, std::min((R - 1 + own - 1) / own, (R - 1) / 4));
+        const int need = std::max((R - 1) * s.segP, P * s.segR);
+        s.threads = (need + 31) / 32 * 32;
+        if (s.threads <= CG_MAXT) return true;
+    }
+    return false;
+}
+
+}  // namespace
+
+int conv_staged_check(int P, int R)
+{
+    if (P < 11 || R < 11) return VERB_ERR_SIZE;
+    int dev = 0, maxsm = 0;
+    StagedShape s;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (cg_smem(P, R) > (size_t)maxsm || !cg_shape(P, R, s)) return VERB_ERR_SIZE;
+    return VERB_OK;
+}
+
+size_t conv_staged_scratch_doubles(int P, int R) { return (cg_scratch(P, R) + 1) & ~(size_t)1; }
+
+int conv_staged_ctas(int P, int R)
+{
+    int dev = 0, sms = 0, per = 0;
+    StagedShape s;
+    if (!cg_shape(P, R, s)) return 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const auto fn = convection_staged_kernel<CG_MAXT, CG_MINB>;
+    allow_max_dynamic_smem((const void*)fn);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, s.threads, cg_smem(P, R));
+    return sms * std::max(per, 1);
+}
+
+void launch_convection_staged(const ConvArgs& a, int nctas, cudaStream_t st)
+{
+    StagedShape s;
+    cg_shape(a.d.P, a.d.R, s);
+    const auto fn = convection_staged_kernel<CG_MAXT, CG_MINB>;
+    allow_max_dynamic_smem((const void*)fn);
+    fn<<<nctas, s.threads, cg_smem(a.d.P, a.d.R), st>>>(a, s.segP, s.segR);
+}
+
+}  // namespace verb

@@ -337,8 +337,11 @@ int conv_run(verb_ctx* c, double dt)
         int s = need_bc(c, b);
         if (s) return s;
     }
-    // the streaming kernel needs both sweeps; other shapes run the contracted
-    // kernel of convection.cu
+    // stream mode: the two-stage kernel where a slice and its unlimited line fit
+    // the shared memory, else one thread per line; both need both sweeps, other
+    // shapes run the contracted kernel of convection.cu
+    const bool staged =
+        c->conv_arith == VERB_CONV_STREAM && conv_staged_check(d.P, d.R) == VERB_OK;
     const bool stream = c->conv_arith == VERB_CONV_STREAM && conv_stream_check(d.P, d.R) == VERB_OK;
     if (!stream)
         if (int s = (c->conv_arith == VERB_CONV_EXACT ? conv_check : conv_check_fma)(d.P, d.R)) return s;
@@ -346,7 +349,9 @@ int conv_run(verb_ctx* c, double dt)
         c->conv_nctas = std::max(conv_ctas(d.P, d.R), conv_ctas_fma(d.P, d.R));
         // one allocation serves every arithmetic mode of the context
         size_t b = (size_t)c->conv_nctas * conv_scratch_doubles(d.P, d.R);
-        if (conv_stream_check(d.P, d.R) == VERB_OK)
+        if (conv_staged_check(d.P, d.R) == VERB_OK)
+            b = std::max(b, (size_t)conv_staged_ctas(d.P, d.R) * conv_staged_scratch_doubles(d.P, d.R));
+        else if (conv_stream_check(d.P, d.R) == VERB_OK)
             b = std::max(b, (size_t)conv_stream_ctas_max(d.P, d.R) * conv_stream_scratch_doubles(d.P, d.R));
         c->conv_scratch_bytes = b * sizeof(double);
     }
@@ -378,7 +383,9 @@ int conv_run(verb_ctx* c, double dt)
     a.status = c->status;
     PhaseTimer t(c, PH_CONV);
     CK(cudaMemsetAsync(c->ticket, 0, sizeof(int), c->stream));
-    if (stream)
+    if (staged)
+        launch_convection_staged(a, conv_staged_ctas(d.P, d.R), c->stream);
+    else if (stream)
         launch_convection_stream(a, conv_stream_ctas(d.P, d.R), c->stream);
     else if (c->conv_arith == VERB_CONV_EXACT)
         launch_convection(a, c->conv_nctas, c->stream);
@@ -1275,7 +1282,10 @@ int verb_assimilate_radial(verb_ctx* c, const double* obs_host, double dt, doubl
         c->pa_p_index = p_index;
     }
     CK(alloc((void**)&c->obs, npts(c) * sizeof(double)));
-    CK(cudaMemcpyAsync(c->obs, obs_host, npts(c) * sizeof(double), cudaMemcpyHostToDevice,
+    // the observations of the MLT in use only
+    const size_t per_p = (size_t)d.R * d.V * d.K;
+    const size_t o0 = p_index >= 0 ? p_index * per_p : 0, on = p_index >= 0 ? per_p : npts(c);
+    CK(cudaMemcpyAsync(c->obs + o0, obs_host + o0, on * sizeof(double), cudaMemcpyHostToDevice,
                        c->stream));
     KFArgs a{};
     a.d = d;
@@ -1296,7 +1306,7 @@ int verb_assimilate_radial(verb_ctx* c, const double* obs_host, double dt, doubl
     a.p_index = p_index;
     a.status = c->status;
     const int nctas = kf_ctas(d, p_index);
-    const size_t wb = (size_t)nctas * 5 * RR * sizeof(double);
+    const size_t wb = (size_t)nctas * kf_work_doubles(d.R) * sizeof(double);
     if (wb > c->kfwork_bytes) {
         cudaFree(c->kfwork);
         c->kfwork = nullptr;
@@ -1641,13 +1651,15 @@ int verb_estimate_device_bytes(int P, int R, int V, int K, int precision, int re
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         size_t cb = (size_t)2 * sms * conv_scratch_doubles(P, R);
-        if (conv_stream_check(P, R) == VERB_OK)
+        if (conv_staged_check(P, R) == VERB_OK)
+            cb = std::max(cb, (size_t)conv_staged_ctas(P, R) * conv_staged_scratch_doubles(P, R));
+        else if (conv_stream_check(P, R) == VERB_OK)
             cb = std::max(cb, (size_t)conv_stream_ctas_max(P, R) * conv_stream_scratch_doubles(P, R));
         b += cb * sizeof(double);
     }
     if (kf_columns > 0)
         b += ((size_t)kf_columns * R * R + np) * sizeof(double) +
-             (size_t)2 * 148 * 5 * R * R * sizeof(double);
+             (size_t)kf_ctas(Dims{P, R, V, K}, -1) * kf_work_doubles(R) * sizeof(double);
     *bytes = b;
     return VERB_OK;
 }

@@ -117,6 +117,11 @@ size_t conv_stream_scratch_doubles(int P, int R);
 int conv_stream_ctas(int P, int R);
 int conv_stream_ctas_max(int P, int R);
 void launch_convection_stream(const ConvArgs& a, int nctas, cudaStream_t s);
+// two stages per pass over line segments (convection_staged.cu)
+int conv_staged_check(int P, int R);  // VERB_ERR_SIZE: the shape needs another kernel
+size_t conv_staged_scratch_doubles(int P, int R);
+int conv_staged_ctas(int P, int R);
+void launch_convection_staged(const ConvArgs& a, int nctas, cudaStream_t s);
 void launch_convection_line(double* psd, const double* x, int n, double lbc, double ubc, int lbc_t,
                             int ubc_t, const double* ux, double dt, int* status, cudaStream_t s);
 
@@ -285,6 +290,7 @@ struct KFArgs {
     int* status;
 };
 int kf_ctas(const Dims& d, int p_index);
+size_t kf_work_doubles(int R);  // workspace of a CTA
 void launch_kf(const KFArgs& a, int nctas, cudaStream_t s);
 
 }  // namespace verb
