@@ -16,8 +16,8 @@
 //          Pa = Pf - K H Pf
 // H selects the finite observations of the slice, so H Pf H^T, Pf H^T and
 // H Pf are gathers, not products.  Dense N x N products run as one batched
-// FP64 GEMM launch over the slices of a chunk (64 x 64 output tiles, 4 x 4
-// outputs per thread); matrix powers use binary exponentiation with
+// FP64 GEMM launch over the slices of a chunk (64 x 64 output tiles on the FP64
+// matrix instruction); matrix powers use binary exponentiation with
 // per-slice exponents (slices whose bit is clear sit out the product); the
 // gain solves run one CTA per slice (LU with partial pivoting of the m x m
 // innovation covariance, the rows of Pf H^T as right-hand sides).
@@ -45,21 +45,25 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b)
 // A: M x K (lda), B: K x N (ldb) or, with TB, N x K; batch b -> slice
 // idx[b] (idx null: b) with per-slice strides.
 //
-// Bound by the FP64 pipe.  With 4 x 4 outputs a thread and scalar multiply-
-// adds, eight shared-memory loads stood against every sixteen of them (12 of
-// 37 TFLOP/s); on the matrix instruction a warp's 32 x 32 outputs take eight
-// loads for sixteen instructions of eight multiply-adds a thread, and the next k
-// step's operands are on their way to registers while this one is used.  Every
-// output is still one chain of fused multiply-adds in ascending k: bit-equal
-// to the scalar form.  24 x 25 x 11 x 11, a whole assimilation: 38.9 -> KFMS ms.
-template <bool TB>
-__global__ void __launch_bounds__(GT) bgemm_kernel(BGemm g)
+// Bound by the FP64 pipe.  On the matrix instruction a warp's 32 x 32 outputs
+// take eight shared-memory loads for sixteen instructions of eight multiply-
+// adds a thread (4 x 4 outputs a thread and scalar multiply-adds: sixteen for
+// every eight, 12 of 37 TFLOP/s); the operand tiles of the next two k steps are
+// on their way to shared memory (cp.async; through registers they were waited
+// for at once, 13 TFLOP/s).  Every output is still one chain of fused
+// multiply-adds in ascending k: bit-equal to the scalar form.  A whole
+// assimilation of 24 x 25 x 11 x 11: 38.9 -> 18.8 ms.
+// VEC: doubles a copy takes (2 where the rows are 16-byte aligned).
+constexpr int GS = 3;  // tiles in flight or in use
+template <bool TB, int VEC>
+__global__ void __launch_bounds__(GT, 3) bgemm_kernel(BGemm g)
 {
-    // k-contiguous rows of 16 + 4: a 4 x 4 operand read fills the banks once
-    __shared__ __align__(16) double As[2][BT][BK + 4];
-    // B by columns like A, or as it is stored, rows of 64 + 4
-    constexpr int BR = TB ? BT : BK, BC = TB ? BK + 4 : BT + 4;
-    __shared__ __align__(16) double Bs[2][BR][BC];
+    // rows of 16 + 4 (A, and B by columns) or of 64 + 4 (B as it is stored):
+    // a 4 x 4 operand read fills the banks once
+    constexpr int AP = BK + 4, BR = TB ? BT : BK, BP = TB ? BK + 4 : BT + 4;
+    extern __shared__ __align__(16) double sm[];
+    double* As = sm;                      // [GS][BT][AP]
+    double* Bs = As + GS * BT * AP;       // [GS][BR][BP]
     const int s = g.idx ? g.idx[blockIdx.z] : blockIdx.z;
     const double* A = g.A + (size_t)s * g.sA;
     const double* B = g.B + (size_t)s * g.sB;
@@ -74,61 +78,65 @@ __global__ void __launch_bounds__(GT) bgemm_kernel(BGemm g)
     for (int r = 0; r < 4; r++)
 #pragma unroll
         for (int c = 0; c < 4; c++) acc[r][c][0] = acc[r][c][1] = 0.0;
-    constexpr int PER = BT * BK / GT;  // elements of a tile a thread stages
-    double ra[PER], rb[PER];
-    auto fetch = [&](int k0) {
-#pragma unroll
-        for (int e = 0; e < PER; e++) {
-            const int t = threadIdx.x + e * GT;
-            const int r = t / BK, k = t % BK;
-            const int gi = i0 + r, gk = k0 + k;
-            double v = 0.0;
-            if (gi < g.M && gk < g.K) {
-                v = A[(size_t)gi * g.lda + gk];
-                if (dk) v = v * dk[gk];
-            }
-            ra[e] = v;
-            v = 0.0;
-            if (TB) {
-                const int gj = j0 + r;
-                if (gk < g.K && gj < g.N) v = B[(size_t)gj * g.ldb + gk];
-            } else {
-                const int kk = k0 + t / BT, gj = j0 + t % BT;
-                if (kk < g.K && gj < g.N) v = B[(size_t)kk * g.ldb + gj];
-            }
-            rb[e] = v;
-        }
+    // a copy of VEC doubles, zero past `have`
+    auto copy = [&](double* dst, const double* src, int have) {
+        const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+        const int bytes = 8 * max(0, min(VEC, have));
+        if (VEC == 2)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes));
+        else
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(bytes));
     };
-    auto stage = [&](int p) {
+    auto fetch = [&](int k0, int p) {
+        if (k0 < g.K) {
+            double* as = As + p * BT * AP;
+            double* bs = Bs + p * BR * BP;
 #pragma unroll
-        for (int e = 0; e < PER; e++) {
-            const int t = threadIdx.x + e * GT;
-            As[p][t / BK][t % BK] = ra[e];
-            Bs[p][TB ? t / BK : t / BT][TB ? t % BK : t % BT] = rb[e];
+            for (int e = 0; e < BT * BK / (GT * VEC); e++) {
+                const int t = (threadIdx.x + e * GT) * VEC;
+                const int r = t / BK, k = t % BK, gi = i0 + r, gk = k0 + k;
+                const int have = gi < g.M ? g.K - gk : 0;
+                copy(as + r * AP + k, have > 0 ? A + (size_t)gi * g.lda + gk : A, have);
+            }
+#pragma unroll
+            for (int e = 0; e < BT * BK / (GT * VEC); e++) {
+                const int t = (threadIdx.x + e * GT) * VEC;
+                const int r = TB ? t / BK : t / BT, c = TB ? t % BK : t % BT;
+                const int gr = TB ? j0 + r : k0 + r, gc = TB ? k0 + c : j0 + c;
+                const int have = gr < (TB ? g.N : g.K) ? (TB ? g.K : g.N) - gc : 0;
+                copy(bs + r * BP + c, have > 0 ? B + (size_t)gr * g.ldb + gc : B, have);
+            }
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    fetch(0);
-    stage(0);
-    __syncthreads();
+    fetch(0, 0);
+    fetch(BK, 1);
     int p = 0;
-    for (int k0 = 0; k0 < g.K; k0 += BK, p ^= 1) {
-        const bool more = k0 + BK < g.K;
-        if (more) fetch(k0 + BK);
+    for (int k0 = 0; k0 < g.K; k0 += BK) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        fetch(k0 + 2 * BK, p + 2 >= GS ? p + 2 - GS : p + 2);
+        const double* as = As + p * BT * AP;
+        const double* bs = Bs + p * BR * BP;
 #pragma unroll
         for (int k = 0; k < BK; k += 4) {
             double a[4], b[4];
 #pragma unroll
-            for (int r = 0; r < 4; r++) a[r] = As[p][wi + 8 * r + gq][k + h];
+            for (int r = 0; r < 4; r++) a[r] = as[(wi + 8 * r + gq) * AP + k + h];
+            if (dk) {
+                const double v = k0 + k + h < g.K ? dk[k0 + k + h] : 0.0;
+#pragma unroll
+                for (int r = 0; r < 4; r++) a[r] = a[r] * v;
+            }
 #pragma unroll
             for (int c = 0; c < 4; c++)
-                b[c] = TB ? Bs[p][wj + 8 * c + gq][k + h] : Bs[p][k + h][wj + 8 * c + gq];
+                b[c] = TB ? bs[(wj + 8 * c + gq) * BP + k + h] : bs[(k + h) * BP + wj + 8 * c + gq];
 #pragma unroll
             for (int r = 0; r < 4; r++)
 #pragma unroll
                 for (int c = 0; c < 4; c++) dmma(acc[r][c], a[r], b[c]);
         }
-        if (more) stage(p ^ 1);
-        __syncthreads();
+        p = p + 1 == GS ? 0 : p + 1;
     }
 #pragma unroll
     for (int r = 0; r < 4; r++)
@@ -249,17 +257,18 @@ __global__ void kc_qdiag_kernel(KCArgs a, double* Q, size_t sQ)
 // Pa = 5 model_error I where it is all zero (first use)
 __global__ void kc_pa_init_kernel(KCArgs a, double* Pa, size_t sPa)
 {
-    __shared__ int any;
     const int b = blockIdx.x;
     const int N = a.d.P * a.d.R;
     double* p = Pa + (size_t)(a.s0 + b) * sPa;
-    if (threadIdx.x == 0) any = 0;
-    __syncthreads();
-    int loc = 0;
-    for (size_t e = threadIdx.x; e < (size_t)N * N; e += blockDim.x)
-        if (p[e] != 0.0) loc = 1;
-    if (loc) any = 1;
-    __syncthreads();
+    // set after the first update: the first values tell
+    int any = 0;
+    const size_t NN = (size_t)N * N, step = 4 * (size_t)blockDim.x;
+    for (size_t e0 = 0; e0 < NN && !any; e0 += step) {
+        int loc = 0;
+        for (size_t e = e0 + threadIdx.x; e < min(NN, e0 + step); e += blockDim.x)
+            if (p[e] != 0.0) loc = 1;
+        any = __syncthreads_or(loc);
+    }
     if (!any)
         for (int i = threadIdx.x; i < N; i += blockDim.x) p[(size_t)i * N + i] = 5 * a.model_error;
 }
@@ -447,13 +456,31 @@ inline unsigned gridx(size_t n, int per = 256, unsigned cap = 64) {
 
 }  // namespace
 
-void launch_bgemm(const BGemm& g, bool tb, int batch, cudaStream_t s)
+namespace {
+
+template <bool TB, int VEC>
+void launch_bgemm_t(const BGemm& g, int batch, cudaStream_t s)
 {
     dim3 grid((g.N + BT - 1) / BT, (g.M + BT - 1) / BT, batch);
-    if (tb)
-        bgemm_kernel<true><<<grid, GT, 0, s>>>(g);
-    else
-        bgemm_kernel<false><<<grid, GT, 0, s>>>(g);
+    const size_t smem = GS * (BT * (BK + 4) + (TB ? BT * (BK + 4) : BK * (BT + 4))) * sizeof(double);
+    allow_max_dynamic_smem((const void*)bgemm_kernel<TB, VEC>);
+    bgemm_kernel<TB, VEC><<<grid, GT, smem, s>>>(g);
+}
+
+}  // namespace
+
+void launch_bgemm(const BGemm& g, bool tb, int batch, cudaStream_t s)
+{
+    // 16-byte copies where every row of every slice starts on 16 bytes
+    const bool even = g.lda % 2 == 0 && g.ldb % 2 == 0 && g.sA % 2 == 0 && g.sB % 2 == 0 &&
+                      (uintptr_t)g.A % 16 == 0 && (uintptr_t)g.B % 16 == 0;
+    if (tb) {
+        if (even) launch_bgemm_t<true, 2>(g, batch, s);
+        else launch_bgemm_t<true, 1>(g, batch, s);
+    } else {
+        if (even) launch_bgemm_t<false, 2>(g, batch, s);
+        else launch_bgemm_t<false, 1>(g, batch, s);
+    }
 }
 
 void launch_kc_split(const KCArgs& a, int nb, int* nt, cudaStream_t s)
