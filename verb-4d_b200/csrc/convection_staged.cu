@@ -1,7 +1,9 @@
 // Convection in (MLT, L) on every (V,K) slice, a QUICKEST pass in two stages
 // over line segments: Convection_2D (src/Convection_2D.cpp:36-169) over
-// Convection_1D_ULTIMATE_QUICKEST6 (QUICKEST6.cpp:22-482), contracted like
-// convection_stream.cu, whose face polynomial, limiter and tables it shares.
+// Convection_1D_ULTIMATE_QUICKEST6 (QUICKEST6.cpp:22-482).  Compiled twice:
+// with multiply-add contraction (stream mode), and with -fmad=false and
+// -DVERB_BUILD_CONV_EXACT, which keeps the reference's operations and their
+// order one by one (bit-identical to it, exp() of loss rates aside).
 //
 // A CTA keeps one [P][R] slice in shared memory for all of its CFL sub-steps.
 // The reference's four loops over a line become two, each run by one thread
@@ -17,23 +19,38 @@
 // stage 2, it keeps in registers from stage 1.
 //
 // What bounds it: the issue of about 240 instructions a face (a third of them
-// FP64), with 16 warps on an SM.  The streaming kernel (one thread a line, all
-// four loops at once) holds some 40 values in flight, which limits it to 12
-// warps whose chains run along the whole line, so a slice of many sub-steps
-// takes as long as its lines are: 24 x 25 x 31 x 31 alone 9.9 ms, 3.4 here
-// (three runs at once 3.78 -> 1.18 ms each); 48 x 101 x 101 x 16 alone 47.4 ms,
-// 23.2 here (one after the other 31.0 -> 23.1 ms).  What the groups and layouts
-// below measured at the latter size is said beside them.
-#include "conv_stream.cuh"
+// FP64; 400 in the exact form), with 16 warps on an SM.  The streaming kernel
+// (one thread a line, all four loops at once) holds some 40 values in flight,
+// which limits it to 12 warps whose chains run along the whole line, so a slice
+// of many sub-steps takes as long as its lines are: 24 x 25 x 31 x 31 alone 9.9
+// ms, 2.7 here; 48 x 101 x 101 x 16 alone 47.4 ms, 23.2 here (one after the other
+// 31.0 -> 23.1 ms).
+#include "quickest.cuh"
 #include "verb_internal.cuh"
 
 #include <algorithm>
 
+#ifdef VERB_BUILD_CONV_EXACT
+#define VERB_STAGED_NS conv_staged_exact
+#define VERB_STAGED(name) name##_exact
+#else
+#define VERB_STAGED_NS conv_staged
+#define VERB_STAGED(name) name
+#endif
+
 namespace verb {
+namespace VERB_STAGED_NS {  // the two compilations keep their kernels apart
 namespace {
 
 constexpr double CG_MAX_SUBSTEPS = 1.0e6;
 constexpr int CG_MAX_OWN = 25;  // cells of a segment: own + 7 flag bits in a word
+
+// the exact form's L sweep divides by G and keeps exp(Loss dt) apart
+#ifdef VERB_BUILD_CONV_EXACT
+constexpr int CG_TABS = 7;
+#else
+constexpr int CG_TABS = 5;
+#endif
 
 // The planes carry CG_GH ghost cells around the slice, so that a window never
 // needs to ask where the line ends.
@@ -51,7 +68,7 @@ struct StagedShape {
 // past a line's end
 __host__ __device__ inline size_t cg_scratch(int P, int R)
 {
-    return 2 * (size_t)P * (R - 1) + 5 * (size_t)P * R + 4 * (size_t)(R - 1) + 4 * (size_t)P +
+    return 2 * (size_t)P * (R - 1) + CG_TABS * (size_t)P * R + 4 * (size_t)(R - 1) + 4 * (size_t)P +
            32 * (size_t)(P > R ? P : R);
 }
 
@@ -78,7 +95,9 @@ struct Seg {
     const double* ln;    // line data (lbc, ubc, dxl, dxu) at ln[i * nl]
     int nl;
     const double *cr, *rc;  // c and 1 / |c| (0 for |c| <= 1e-31) of face k at [k * nl]
-    const double *e1, *e2;  // store epilogue of cell k: times e1, plus e2 (or nullptr)
+    // store epilogue of cell k: times e1 (P), or: times e1 plus e2 (R); the
+    // exact form divides by e3 (reciprocal e4) before, in the L sweep
+    const double *e1, *e2, *e3, *e4;
 };
 
 // ghost cells of the line before a pass (:89-143)
@@ -104,13 +123,45 @@ __device__ __forceinline__ void line_ghosts(double* E, int st, int n, int lt, in
     }
 }
 
-// Stage 1 takes the faces of a segment CG_U at a time, stage 2 CG_W: the
+// Stage 1 takes the faces of a segment U at a time, stage 2 three: the
 // polynomials and the limiters of a group are independent of each other, and
 // the window is loaded once per group instead of shifted through registers.
-// Groups of 6 and 3: 23.2 ms (4 and 4: 28.8, spilling; 12 and 4: 34.0; 6 and 6:
-// 24.3; a window shifted face by face 29.8).
-constexpr int CG_U = 6, CG_W = 3;
 
+#ifdef VERB_BUILD_CONV_EXACT
+// a / b rounded to nearest with y = RN(1/b) (Markstein's correction, as in
+// div_const) for |a|, |b| in [2^-400, 2^400), where neither the quotient nor its
+// residual leaves the normal range; others are divided.
+__device__ __forceinline__ double div_by(double a, double b, double y)
+{
+    const double q = a * y;
+    const unsigned ea = ((unsigned)__double2hiint(a) & 0x7fffffffu) - 0x26f00000u;
+    const unsigned eb = ((unsigned)__double2hiint(b) & 0x7fffffffu) - 0x26f00000u;
+    if (eb < 0x32000000u) {
+        if (ea < 0x32000000u) return fma(fma(-q, b, a), y, q);
+        if (a == 0.0) return q;
+    }
+    return a / b;
+}
+
+// Unlimited values of U faces from the window d[k] = E[x-5+k], the roles of the
+// stencil's points chosen by the direction (QUICKEST6.cpp:169-186)
+template <int U>
+__device__ __forceinline__ void faces(double (&d)[U + 9], const double (&c)[U], double (&f)[U])
+{
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const bool pos = c[u] >= 0;
+        double a[5], b[5];  // upwind from the centre on, downwind
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            a[k] = pos ? d[u + 4 - k] : d[u + 5 + k];
+            b[k] = pos ? d[u + 5 + k] : d[u + 4 - k];
+        }
+        const FaceCoef k = face_coef_exact(c[u]);
+        f[u] = quickest_face_k(a[1], a[2], a[3], a[4], a[0], b[0], b[1], b[2], b[3], b[4], c[u], k);
+    }
+}
+#else
 // Unlimited values of U faces from the window d[k] = E[x-5+k] (QUICKEST6.cpp:
 // 162-241, in the positive orientation with the signed Courant number).  The
 // differences of the stencil are built level by level for all of the group's
@@ -166,10 +217,12 @@ __device__ __forceinline__ void faces(double (&d)[U + 9], const double (&c)[U], 
         f[u] += (p[u] * (1.0 / 362880.0)) * (c[u] >= 0 ? d[u] : d[u + 1]);
 }
 
+#endif
+
 // returns unlimited face a, whose slot is the neighbour's
+template <int U>
 __device__ __forceinline__ double stage1(const Seg& L)
 {
-    constexpr int U = CG_U;
     double Q = 0.0, f0 = 0.0;
     const double* cp = L.cr + L.a * L.nl;
     // faces a .. a+own, cells a .. a+own-1; what is read past the line's
@@ -255,11 +308,17 @@ __device__ __forceinline__ double limit(double f, double c, double rc, double em
     const double od = pos ? e0 : em1;
     const double DEL = od - ou;
     const double CURV = od - 2 * oc + ou;
-    // not flat implies DEL != 0 (where it is NaN, so is f and what follows)
     const bool flat = fabs(CURV) >= fabs(DEL);
-    const bool useref = !peak & !flat & (__double2hiint(rc) != 0);
+    const bool rise = DEL > 0, fall = DEL < 0;
+    const bool useref = !peak & !flat & (__double2hiint(rc) != 0) & (rise | fall);
+#ifdef VERB_BUILD_CONV_EXACT
+    const double ref = ou + div_by(oc - ou, fabs(c), rc);
+#else
     const double ref = ou + (oc - ou) * rc;
-    const int s = DEL > 0 ? 0 : (int)0x80000000;
+#endif
+    // max and min as selects that keep fmax's and fmin's values where f, oc or
+    // ref is not a number (ou and od are numbers here)
+    const int s = rise ? 0 : (int)0x80000000;
     const double a = flip(f, s), lo = flip(oc, s), h1 = flip(ref, s), h2 = flip(od, s);
     double t = a > lo ? a : lo;
     const double hi = h1 < h2 ? h1 : h2;
@@ -267,6 +326,16 @@ __device__ __forceinline__ double limit(double f, double c, double rc, double em
     double res = useref ? flip(t, s) : f;
     if (!peak & flat) res = oc;
     return res;
+}
+
+// v h1 + h2, for the exact form's L sweep (v / h3) h1 + h2 (h4 = RN(1 / h3))
+__device__ __forceinline__ double epilogue(double v, double h1, double h2, double h3, double h4,
+                                           bool div)
+{
+#ifdef VERB_BUILD_CONV_EXACT
+    if (div) v = div_by(v, h3, h4);
+#endif
+    return v * h1 + h2;
 }
 
 // last: the line's last sub-cycle, whose cells take the store epilogue
@@ -307,7 +376,7 @@ __device__ __forceinline__ void stage2(const Seg& L, double f0, bool last)
     // face x takes positions x-4 .. x-2, or x-3 .. x-1 against the direction
     unsigned three = M | M >> 1 | M >> 2;
 
-    constexpr int U = CG_W;
+    constexpr int U = 3;
     double Rp = 0.0, first = 0.0, second = 0.0, end = 0.0;
     int at = L.a * L.nl;
 #pragma unroll 1
@@ -315,12 +384,12 @@ __device__ __forceinline__ void stage2(const Seg& L, double f0, bool last)
         const int x = L.a + i;
         const double* ep = L.E + (x - 2) * L.st;
         double* op = L.O + (x - 1) * L.st;
-        double c[U], rc[U], h1[U], h2[U], w[U + 3], f[U];
+        double c[U], rc[U], h1[U], h2[U], h3[U], h4[U], w[U + 3], f[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
             c[u] = L.cr[at];
             rc[u] = L.rc[at];
-            h1[u] = 1.0;
+            h1[u] = h3[u] = h4[u] = 1.0;
             h2[u] = 0.0;
             at += L.nl;
             // cell x + u - 1 (the first group's entry of cell a - 1, and past
@@ -328,6 +397,12 @@ __device__ __forceinline__ void stage2(const Seg& L, double f0, bool last)
             if (last) {
                 h1[u] = L.e1[at - 2 * L.nl];
                 if (L.e2) h2[u] = L.e2[at - 2 * L.nl];
+#ifdef VERB_BUILD_CONV_EXACT
+                if (L.e2) {
+                    h3[u] = L.e3[at - 2 * L.nl];
+                    h4[u] = L.e4[at - 2 * L.nl];
+                }
+#endif
             }
         }
 #pragma unroll
@@ -341,7 +416,8 @@ __device__ __forceinline__ void stage2(const Seg& L, double f0, bool last)
             const double r = c[u] * limit(f[u], c[u], rc[u], w[u], w[u + 1], w[u + 2], w[u + 3],
                                           peak);
             const double o = w[u + 1] - (r - Rp);
-            if ((u > 0 || i > 0) && i + u <= L.own) op[u * L.st] = o * h1[u] + h2[u];
+            if ((u > 0 || i > 0) && i + u <= L.own)
+                op[u * L.st] = epilogue(o, h1[u], h2[u], h3[u], h4[u], last && L.e2);
             if (u == 1 && i == 0) first = o;
             if (u == 2 && i == 0) second = o;
             if (L.ut == VERB_BC_CONSTANT_DERIVATIVE && i + u == L.own) end = o;
@@ -350,7 +426,12 @@ __device__ __forceinline__ void stage2(const Seg& L, double f0, bool last)
         three >>= U;
     }
     // boundary rewrite (:462-477): the cells at the line's ends (no source term)
-    auto put = [&](int k, double v) { L.O[k * L.st] = last ? v * L.e1[k * L.nl] : v; };
+    auto put = [&](int k, double v) {
+#ifdef VERB_BUILD_CONV_EXACT
+        if (last && L.e2) v = v / L.e3[k * L.nl];
+#endif
+        L.O[k * L.st] = last ? v * L.e1[k * L.nl] : v;
+    };
     if (L.a == 0) {
         if (L.lt == VERB_BC_PERIODIC) put(L.n - 1, first);
         else put(0, L.lt == VERB_BC_CONSTANT_VALUE ? L.ln[0] : second);
@@ -375,7 +456,7 @@ __device__ __forceinline__ double cg_block_max(double v, double* red)
     return m;
 }
 
-template <int MAXT, int MINB>
+template <int U1, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs a, int segP, int segR)
 {
     extern __shared__ __align__(16) double sm[];
@@ -399,9 +480,16 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
     double* e1P = rcP + P1;                    // G
     double* crR = e1P + (size_t)PR;
     double* rcR = crR + (size_t)PR;
-    double* e1R = rcR + (size_t)PR;            // exp(Loss dt)/G
+    double* e1R = rcR + (size_t)PR;            // exp(Loss dt)/G, or exp(Loss dt)
     double* e2R = e1R + (size_t)PR;            // S dt, 0 at the ends
+#ifdef VERB_BUILD_CONV_EXACT
+    double* e3R = e2R + (size_t)PR;            // G
+    double* e4R = e3R + (size_t)PR;            // 1 / G
+    double* lnP = e4R + (size_t)PR;            // [4][R-1]
+#else
+    double *e3R = nullptr, *e4R = nullptr;
     double* lnP = e2R + (size_t)PR;            // [4][R-1]
+#endif
     double* lnR = lnP + 4 * (size_t)(R - 1);   // [4][P]
     const int nslices = V * K;
 
@@ -458,7 +546,13 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
             const size_t gi = g(iP, iR);
             const double G = a.G[gi];
             if (iR < R - 1) e1P[(size_t)iP * (R - 1) + iR] = G;
+#ifdef VERB_BUILD_CONV_EXACT
+            e1R[(size_t)iR * P + iP] = exp(a.loss[gi] * dtc);
+            e3R[(size_t)iR * P + iP] = G;
+            e4R[(size_t)iR * P + iP] = __drcp_rn(G);
+#else
             e1R[(size_t)iR * P + iP] = exp(a.loss[gi] * dtc) / G;
+#endif
             e2R[(size_t)iR * P + iP] = iR && iR < R - 1 ? a.S[gi] * dtc : 0.0;
         }
         // per-line CFL sub-cycles and face Courant numbers (QUICKEST6.cpp:37-52,
@@ -541,6 +635,8 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
                 L.rc = (pr ? rcP : rcR) + line;
                 L.e1 = (pr ? e1P : e1R) + line;
                 L.e2 = pr ? nullptr : e2R + line;
+                L.e3 = e3R + line;
+                L.e4 = e4R + line;
                 const int ns = live ? (pr ? nsP : nsR)[line] : 0;
                 // the line's own CFL sub-cycles (:37-52), the epilogue on the
                 // last one only
@@ -555,7 +651,7 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
                     const bool run = k < ns, last = k == ns - 1;
                     double f0 = 0.0;
                     __syncthreads();
-                    if (run) f0 = stage1(L);
+                    if (run) f0 = stage1<U1>(L);
                     __syncthreads();
                     if (run) {
                         stage2(L, f0, last);
@@ -584,17 +680,42 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
     }
 }
 
-constexpr int CG_MAXT = 512;  // 125 registers a thread
-constexpr int CG_MINB = 1;
+// Launch shapes: cells of a segment, longer where the lines would need more
+// threads than a CTA has, and the kernel for that many threads.
+//
+// Contracted form.  11 cells, 512 threads (125 registers; stage 1 in groups of 6:
+// 23.2 ms at 48 x 101 x 101 x 16, of 4 28.8, of 12 34.0, spilling; a window shifted
+// face by face 29.8).  Below 1200 points a pass waits for the slices of the most
+// sub-steps: 5 cells and two slices on an SM, 24 x 25 x 31 x 31 alone (and per
+// pass of three runs at once) 2.7 (1.08) ms, against 2.8 (1.14) with four
+// slices, 2.2 (2.22) with 2 cells and one slice.
+//
+// Exact form, one slice on an SM at a time.  Alone (and per pass of three runs
+// at once), line-job kernel before the arrow: 12 x 13 x 31 x 31, 2 cells 1.11 (0.70)
+// -> 1.20 (0.54) ms; 24 x 25 x 31 x 31, 5 cells 4.00 (2.59) -> 3.60 (1.82), with 2
+// cells 3.42 (3.40), 8 cells 4.80 (2.48); 13 x 90 x 31 x 31, 8 cells 3.68 (2.55) ->
+// 3.57 (2.43), 5 cells 2.98 (2.91); 24 x 51 x 31 x 31, 8 cells 6.69 (4.34) -> 6.03
+// (4.16); 48 x 51 x 45 x 21, 5 cells (and up to 512 threads) 23.5 (14.9) -> 13.9
+// (13.6); 48 x 101 x 61 x 13 40.7 (21.7) -> 24.4 (20.4).  With two slices on an SM
+// the slices of the most sub-steps slow each other: 24 x 51 alone 7.5 ms.
+constexpr int CG_MAXT = 512;
+#ifdef VERB_BUILD_CONV_EXACT
+int cg_own(int P, int R)
+{
+    const int n = P * R;
+    return n < 400 ? 2 : (n >= 1000 && n < 1800 ? 8 : 5);
+}
+constexpr int CG_STEP = 3, CG_RESIDENT = 1;
+#else
+int cg_own(int P, int R) { return P * R < 1200 ? 5 : 11; }
+constexpr int CG_STEP = 6, CG_RESIDENT = 32;
+#endif
 
-// Segments whose faces fill whole groups: of 5 cells on small slices, where a
-// sub-step's chain is what a pass waits for, of 11 on others, longer where the
-// lines would need more threads than a CTA has.
 bool cg_shape(int P, int R, StagedShape& s)
 {
-    for (int own = P * R < 1200 ? CG_U - 1 : 2 * CG_U - 1; own <= CG_MAX_OWN; own += CG_U) {
-        s.segP = std::max(1, std::min((P - 1 + own - 1) / own, (P - 1) / 4));
-        s.segR = std::max(1, std::min((R - 1 + own - 1) / own, (R - 1) / 4));
+    for (int own = cg_own(P, R); own <= CG_MAX_OWN; own += CG_STEP) {
+        s.segP = (P - 1 + own - 1) / own;
+        s.segR = (R - 1 + own - 1) / own;
         const int need = std::max((R - 1) * s.segP, P * s.segR);
         s.threads = (need + 31) / 32 * 32;
         if (s.threads <= CG_MAXT) return true;
@@ -602,9 +723,27 @@ bool cg_shape(int P, int R, StagedShape& s)
     return false;
 }
 
-}  // namespace
+typedef void (*StagedKernel)(ConvArgs, int, int);
+StagedKernel cg_kernel(int P, int R, const StagedShape& s)
+{
+#ifdef VERB_BUILD_CONV_EXACT
+    StagedKernel fn = convection_staged_kernel<3, CG_MAXT, 1>;
+    if (s.threads <= 320) fn = convection_staged_kernel<3, 320, 1>;
+    if (s.threads <= 160) fn = convection_staged_kernel<3, 160, 2>;
+#else
+    StagedKernel fn = convection_staged_kernel<6, CG_MAXT, 1>;
+    if (P * R < 1200 && s.threads <= 160) fn = convection_staged_kernel<3, 160, 2>;
+#endif
+    allow_max_dynamic_smem((const void*)fn);
+    return fn;
+}
 
-int conv_staged_check(int P, int R)
+}  // namespace
+}  // namespace VERB_STAGED_NS
+
+using namespace VERB_STAGED_NS;
+
+int VERB_STAGED(conv_staged_check)(int P, int R)
 {
     if (P < 11 || R < 11) return VERB_ERR_SIZE;
     int dev = 0, maxsm = 0;
@@ -615,27 +754,25 @@ int conv_staged_check(int P, int R)
     return VERB_OK;
 }
 
-size_t conv_staged_scratch_doubles(int P, int R) { return (cg_scratch(P, R) + 1) & ~(size_t)1; }
+size_t VERB_STAGED(conv_staged_scratch_doubles)(int P, int R) { return (cg_scratch(P, R) + 1) & ~(size_t)1; }
 
-int conv_staged_ctas(int P, int R)
+int VERB_STAGED(conv_staged_ctas)(int P, int R)
 {
     int dev = 0, sms = 0, per = 0;
     StagedShape s;
     if (!cg_shape(P, R, s)) return 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const auto fn = convection_staged_kernel<CG_MAXT, CG_MINB>;
-    allow_max_dynamic_smem((const void*)fn);
+    const StagedKernel fn = cg_kernel(P, R, s);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, s.threads, cg_smem(P, R));
-    return sms * std::max(per, 1);
+    return sms * std::min(std::max(per, 1), CG_RESIDENT);
 }
 
-void launch_convection_staged(const ConvArgs& a, int nctas, cudaStream_t st)
+void VERB_STAGED(launch_convection_staged)(const ConvArgs& a, int nctas, cudaStream_t st)
 {
     StagedShape s;
     cg_shape(a.d.P, a.d.R, s);
-    const auto fn = convection_staged_kernel<CG_MAXT, CG_MINB>;
-    allow_max_dynamic_smem((const void*)fn);
+    const StagedKernel fn = cg_kernel(a.d.P, a.d.R, s);
     fn<<<nctas, s.threads, cg_smem(a.d.P, a.d.R), st>>>(a, s.segP, s.segR);
 }
 

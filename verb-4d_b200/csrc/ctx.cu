@@ -320,6 +320,23 @@ int local_run(verb_ctx* c, double dt, double sub_dt)
     return check_launch();
 }
 
+// Bytes of the slice tables of a context's convection: one allocation serves
+// every arithmetic mode, with no more CTAs than slices.
+size_t conv_scratch_size(const Dims& d)
+{
+    const size_t slices = (size_t)d.V * d.K;
+    auto ctas = [&](int n) { return std::min<size_t>(n, slices); };
+    const int P = d.P, R = d.R;
+    size_t b = ctas(std::max(conv_ctas(P, R), conv_ctas_fma(P, R))) * conv_scratch_doubles(P, R);
+    if (conv_staged_check_exact(P, R) == VERB_OK)
+        b = std::max(b, ctas(conv_staged_ctas_exact(P, R)) * conv_staged_scratch_doubles_exact(P, R));
+    if (conv_staged_check(P, R) == VERB_OK)
+        b = std::max(b, ctas(conv_staged_ctas(P, R)) * conv_staged_scratch_doubles(P, R));
+    else if (conv_stream_check(P, R) == VERB_OK)
+        b = std::max(b, ctas(conv_stream_ctas_max(P, R)) * conv_stream_scratch_doubles(P, R));
+    return b * sizeof(double);
+}
+
 int conv_run(verb_ctx* c, double dt)
 {
     const Dims& d = c->d;
@@ -337,23 +354,20 @@ int conv_run(verb_ctx* c, double dt)
         int s = need_bc(c, b);
         if (s) return s;
     }
-    // stream mode: the two-stage kernel where a slice and its unlimited line fit
-    // the shared memory, else one thread per line; both need both sweeps, other
-    // shapes run the contracted kernel of convection.cu
-    const bool staged =
-        c->conv_arith == VERB_CONV_STREAM && conv_staged_check(d.P, d.R) == VERB_OK;
+    // the two-stage kernel where both sweeps run and a slice's planes fit the
+    // shared memory; other shapes take one thread per line (stream mode) or
+    // the line-job kernels of convection.cu
+    const bool staged = c->conv_arith == VERB_CONV_STREAM ? conv_staged_check(d.P, d.R) == VERB_OK
+                        : c->conv_arith == VERB_CONV_EXACT
+                            ? conv_staged_check_exact(d.P, d.R) == VERB_OK : false;
     const bool stream = c->conv_arith == VERB_CONV_STREAM && conv_stream_check(d.P, d.R) == VERB_OK;
     if (!stream)
         if (int s = (c->conv_arith == VERB_CONV_EXACT ? conv_check : conv_check_fma)(d.P, d.R)) return s;
+    // no more CTAs than slices
+    auto cap = [&](int ctas) { return (int)std::min<size_t>(ctas, (size_t)d.V * d.K); };
     if (!c->conv_nctas) {
-        c->conv_nctas = std::max(conv_ctas(d.P, d.R), conv_ctas_fma(d.P, d.R));
-        // one allocation serves every arithmetic mode of the context
-        size_t b = (size_t)c->conv_nctas * conv_scratch_doubles(d.P, d.R);
-        if (conv_staged_check(d.P, d.R) == VERB_OK)
-            b = std::max(b, (size_t)conv_staged_ctas(d.P, d.R) * conv_staged_scratch_doubles(d.P, d.R));
-        else if (conv_stream_check(d.P, d.R) == VERB_OK)
-            b = std::max(b, (size_t)conv_stream_ctas_max(d.P, d.R) * conv_stream_scratch_doubles(d.P, d.R));
-        c->conv_scratch_bytes = b * sizeof(double);
+        c->conv_nctas = cap(std::max(conv_ctas(d.P, d.R), conv_ctas_fma(d.P, d.R)));
+        c->conv_scratch_bytes = conv_scratch_size(d);
     }
     CK(alloc((void**)&c->conv_scratch, c->conv_scratch_bytes));
     CK(alloc((void**)&c->conv_substeps, (size_t)d.V * d.K * sizeof(int)));
@@ -383,10 +397,12 @@ int conv_run(verb_ctx* c, double dt)
     a.status = c->status;
     PhaseTimer t(c, PH_CONV);
     CK(cudaMemsetAsync(c->ticket, 0, sizeof(int), c->stream));
-    if (staged)
-        launch_convection_staged(a, conv_staged_ctas(d.P, d.R), c->stream);
+    if (staged && c->conv_arith == VERB_CONV_EXACT)
+        launch_convection_staged_exact(a, cap(conv_staged_ctas_exact(d.P, d.R)), c->stream);
+    else if (staged)
+        launch_convection_staged(a, cap(conv_staged_ctas(d.P, d.R)), c->stream);
     else if (stream)
-        launch_convection_stream(a, conv_stream_ctas(d.P, d.R), c->stream);
+        launch_convection_stream(a, cap(conv_stream_ctas(d.P, d.R)), c->stream);
     else if (c->conv_arith == VERB_CONV_EXACT)
         launch_convection(a, c->conv_nctas, c->stream);
     else
@@ -1647,15 +1663,7 @@ int verb_estimate_device_bytes(int P, int R, int V, int K, int precision, int re
         if (refinements > 0) b += 2 * np * sizeof(double);
     }
     if (P >= 3 || R >= 3) {
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        size_t cb = (size_t)2 * sms * conv_scratch_doubles(P, R);
-        if (conv_staged_check(P, R) == VERB_OK)
-            cb = std::max(cb, (size_t)conv_staged_ctas(P, R) * conv_staged_scratch_doubles(P, R));
-        else if (conv_stream_check(P, R) == VERB_OK)
-            cb = std::max(cb, (size_t)conv_stream_ctas_max(P, R) * conv_stream_scratch_doubles(P, R));
-        b += cb * sizeof(double);
+        b += conv_scratch_size(Dims{P, R, V, K});
     }
     if (kf_columns > 0)
         b += ((size_t)kf_columns * R * R + np) * sizeof(double) +
