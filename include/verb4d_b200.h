@@ -257,7 +257,8 @@ int verb_local_solve_variant(int v, int* warps_per_cta, int* l_columns, int* u_c
  * the window lives in shared memory.  Bands wider than the register window
  * holds (V > 126) fall back to the shared-memory window. */
 int verb_local_solve_variant_window(int v, int* in_registers);
-/* v = -1: the shape tuned for this context's shape in this process (else 0) */
+/* v = -1: the shape tuned for this context's shape in this process, else one
+ * chosen by the number and the band of its systems */
 int verb_set_local_solve_variant(verb_ctx* ctx, int v);
 int verb_autotune_local_solve(verb_ctx* ctx, double dt, double sub_dt, double* times_ms,
                               int* chosen);

@@ -162,7 +162,7 @@ int solve_variant_for(verb_ctx* c)
     if (c->solve_variant >= 0) return c->solve_variant;
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tuned_solve.find(tune_key(c));
-    return it == g_tuned_solve.end() ? 0 : it->second;
+    return it == g_tuned_solve.end() ? -1 : it->second;  // -1: launch_local_solve's rule
 }
 
 int local_prepare(verb_ctx* c, LocalArgs& a, double dts)

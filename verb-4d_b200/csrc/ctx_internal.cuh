@@ -106,7 +106,7 @@ struct verb_ctx {
     float *kpfeat = nullptr, *kpc = nullptr;
     bool local_dirty = true;
     double local_dt = -1;
-    int solve_variant = -1;  // local solve shape; -1: the process-wide tuned one, else 0
+    int solve_variant = -1;  // local solve shape; -1: the process-wide tuned one, else by rule
     const double* dkv_override = nullptr;  // Dyx for the per-slice entry point
     // convection
     double* conv_scratch = nullptr;

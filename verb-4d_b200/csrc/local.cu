@@ -2155,12 +2155,37 @@ void local_solve_variant_shape(int v, int* warps, int* fwd, int* bwd, int* rw)
     if (rw) *rw = sh.rw;
 }
 
+// The shape a context takes that was not tuned.  One system per CTA with 16 L
+// and 12 U columns in flight has the shortest column chain as long as the
+// systems come in at most two waves (its ring leaves 11 resident on an SM at V =
+// 101 in FP64): 24 x 25 x 31 x 31 0.48 ms against 0.57 for 4 x 4 x 3 and 0.77 for the
+// shared-memory window 4 x 4 x 2, 24 x 51 x 101 x 21 1.39 / 1.56 / 2.48 ms, 48 x 101 x
+// 61 x 12 1.07 / 1.14 / 1.44 ms.  Beyond that shallower rings with more systems
+// resident: 48 x 101 x 101 x 12 2.53 ms (4 x 6 x 4) against 2.77 and 2.98 ms.
+int local_solve_default(const LocalArgs& a)
+{
+    constexpr int deep = 14, wide = 10;
+    static_assert(SOLVE_SHAPES[deep].warps == 1 && SOLVE_SHAPES[deep].fwd == 16 &&
+                      SOLVE_SHAPES[wide].warps == 4 && SOLVE_SHAPES[wide].fwd == 6,
+                  "the shapes the rule names");
+    int dev = 0, sms = 148, smem = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+    const size_t ring = a.factors32
+        ? solve_ring_doubles(a.klp32, a.kvp32, sizeof(float), SOLVE_SHAPES[deep].fwd, SOLVE_SHAPES[deep].bwd)
+        : solve_ring_doubles(a.klp, a.kvp, sizeof(double), SOLVE_SHAPES[deep].fwd, SOLVE_SHAPES[deep].bwd);
+    const long long resident = smem / ((ring + 16) * 8 + 1024);
+    return (long long)a.d.P * a.d.R <= 2 * resident * sms ? deep : wide;
+}
+
 void launch_local_solve(const LocalArgs& a, cudaStream_t s)
 {
+    const int v = a.solve_variant >= 0 ? a.solve_variant : local_solve_default(a);
     if (a.factors32)
-        launch_solve_v<float>(a, a.solve_variant, a.klp32, a.kvp32, s);
+        launch_solve_v<float>(a, v, a.klp32, a.kvp32, s);
     else
-        launch_solve_v<double>(a, a.solve_variant, a.klp, a.kvp, s);
+        launch_solve_v<double>(a, v, a.klp, a.kvp, s);
 }
 
 }  // namespace verb

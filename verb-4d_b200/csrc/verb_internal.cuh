@@ -153,7 +153,8 @@ struct LocalArgs {
     // ConstantValue 0 boundary.  nullptr: every system is the full V*K grid.
     const int* k0;
     const long long* uoff;
-    // local solve shape (local_solve_variant_shape), chosen by the autotuner
+    // local solve shape (local_solve_variant_shape): the autotuner's or the caller's
+    // choice, -1: by size (launch_local_solve)
     int solve_variant;
     // optional per-system selection: only systems with (sel[sys] & sel_mask)
     // != 0 are processed
