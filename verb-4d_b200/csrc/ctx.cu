@@ -17,16 +17,138 @@ size_t bc_elems(const verb_ctx* c, int b)
     }
 }
 
+// Device memory and stream of a per-slice call.  Allocating and freeing them in
+// every call was most of its cost (an allocation and its free take 0.6-0.9 ms, a
+// stream 0.1 ms, the kernels of a 24 x 25 convection slice 0.07 ms), so up to
+// ARENA_KEEP blocks of up to ARENA_BYTES each are kept idle between calls.  A
+// block serves one call at a time (taken and put back under the lock, its
+// stream drained before); idle blocks are given back when an allocation fails
+// and at exit.  What a block has no room for is allocated by itself.
+struct Arena {
+    char* base = nullptr;
+    size_t size = 0, used = 0;
+    int device = -1;
+    cudaStream_t stream = nullptr;
+};
+constexpr size_t ARENA_KEEP = 4, ARENA_BYTES = (size_t)16 << 20;
+std::mutex g_arena_mu;
+std::vector<Arena> g_arenas;          // idle
+thread_local Arena* t_arena = nullptr;  // of the call this thread is in
+
+void arena_free(Arena& a)
+{
+    int dev = -1;
+    cudaGetDevice(&dev);
+    if (a.device >= 0 && a.device != dev) cudaSetDevice(a.device);
+    if (a.stream) cudaStreamDestroy(a.stream);
+    cudaFree(a.base);
+    if (a.device >= 0 && a.device != dev) cudaSetDevice(dev);
+    a = Arena{};
+}
+
+// idle blocks back to the device; true when there were any
+bool arenas_release()
+{
+    std::vector<Arena> idle;
+    {
+        std::lock_guard<std::mutex> lk(g_arena_mu);
+        idle.swap(g_arenas);
+    }
+    for (Arena& a : idle) arena_free(a);
+    return !idle.empty();
+}
+
+int arena_take(Arena& a, size_t bytes)
+{
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    Arena got;
+    {
+        std::lock_guard<std::mutex> lk(g_arena_mu);
+        for (size_t i = g_arenas.size(); i-- > 0;)
+            if (g_arenas[i].device == dev && g_arenas[i].size >= bytes) {
+                got = g_arenas[i];
+                g_arenas.erase(g_arenas.begin() + i);
+                break;
+            }
+    }
+    if (got.base) {
+        // still there (the device may have been reset in between)
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, got.base) == cudaSuccess &&
+            at.type == cudaMemoryTypeDevice && cudaStreamQuery(got.stream) == cudaSuccess) {
+            a = got;
+            a.used = 0;
+            return VERB_OK;
+        }
+        cudaGetLastError();
+    }
+    a = Arena{};
+    a.device = dev;
+    cudaError_t e = cudaMalloc(&a.base, bytes);
+    if (e == cudaErrorMemoryAllocation && arenas_release()) {
+        cudaGetLastError();
+        e = cudaMalloc(&a.base, bytes);
+    }
+    if (e == cudaSuccess) {
+        a.size = bytes;
+        e = cudaStreamCreateWithFlags(&a.stream, cudaStreamNonBlocking);
+    }
+    if (e != cudaSuccess) arena_free(a);
+    return cuda_ok(e);
+}
+
+// the block's work is done
+void arena_put(Arena& a)
+{
+    if (!a.base) return;
+    Arena out = a;
+    a = Arena{};
+    if (out.size <= ARENA_BYTES) {
+        std::lock_guard<std::mutex> lk(g_arena_mu);
+        g_arenas.push_back(out);
+        if (g_arenas.size() <= ARENA_KEEP) return;
+        out = g_arenas.front();
+        g_arenas.erase(g_arenas.begin());
+    }
+    arena_free(out);
+}
+
+struct ArenasAtExit {
+    ~ArenasAtExit() { arenas_release(); }
+} g_arenas_at_exit;
+
+cudaError_t dev_malloc(void** p, size_t bytes)
+{
+    if (t_arena && bytes <= t_arena->size - t_arena->used) {
+        *p = t_arena->base + t_arena->used;
+        t_arena->used += std::min((bytes + 255) & ~(size_t)255, t_arena->size - t_arena->used);
+        return cudaSuccess;
+    }
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && arenas_release()) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
+void dev_free(void* p)
+{
+    if (t_arena && (char*)p >= t_arena->base && (char*)p < t_arena->base + t_arena->size) return;
+    cudaFree(p);
+}
+
 int alloc(void** p, size_t bytes)
 {
     if (*p) return VERB_OK;
-    return cuda_ok(cudaMalloc(p, bytes));
+    return cuda_ok(dev_malloc(p, bytes));
 }
 
 int ensure_field(verb_ctx* c, int fid)
 {
     if (c->f[fid]) return VERB_OK;
-    CK(cudaMalloc(&c->f[fid], npts(c) * sizeof(double)));
+    CK(dev_malloc((void**)&c->f[fid], npts(c) * sizeof(double)));
     return VERB_OK;
 }
 
@@ -53,7 +175,7 @@ int need_field(verb_ctx* c, int fid)
 int need_bc(verb_ctx* c, int b)
 {
     if (c->bc[b]) return VERB_OK;
-    CK(cudaMalloc(&c->bc[b], bc_elems(c, b) * sizeof(double)));
+    CK(dev_malloc((void**)&c->bc[b], bc_elems(c, b) * sizeof(double)));
     CK(cudaMemsetAsync(c->bc[b], 0, bc_elems(c, b) * sizeof(double), c->stream));
     return VERB_OK;
 }
@@ -497,9 +619,9 @@ int verb_create(verb_ctx** out, int P, int R, int V, int K, void* stream)
             c->own_stream = true;
         }
     }
-    if (!st) st = cuda_ok(cudaMalloc(&c->status, sizeof(int)));
+    if (!st) st = cuda_ok(dev_malloc((void**)&c->status, sizeof(int)));
     if (!st) st = cuda_ok(cudaMemsetAsync(c->status, 0, sizeof(int), c->stream));
-    if (!st) st = cuda_ok(cudaMalloc(&c->red, 2 * sizeof(unsigned long long)));
+    if (!st) st = cuda_ok(dev_malloc((void**)&c->red, 2 * sizeof(unsigned long long)));
     if (st) {
         verb_destroy(c);
         return st;
@@ -515,25 +637,25 @@ int verb_destroy(verb_ctx* c)
     if (c->out_stream) cudaStreamDestroy(c->out_stream);
     if (c->out_ev_snap) cudaEventDestroy(c->out_ev_snap);
     if (c->out_ev_host) cudaEventDestroy(c->out_ev_host);
-    cudaFree(c->out_snap);
+    dev_free(c->out_snap);
     cudaFreeHost(c->out_host);
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (int i = 0; i < VERB_F_COUNT; i++) {
-        cudaFree(c->f[i]);
-        cudaFree(c->fbase[i]);
+        dev_free(c->f[i]);
+        dev_free(c->fbase[i]);
         if (c->upd[i]) {
             for (UpdComponent& k : c->upd[i]->comps) {
-                cudaFree(k.base);
-                for (auto& e : k.data_q) cudaFree(e.second);
+                dev_free(k.base);
+                for (auto& e : k.data_q) dev_free(e.second);
             }
             delete c->upd[i];
         }
     }
-    for (int i = 0; i < VERB_BCF_COUNT; i++) cudaFree(c->bc[i]);
+    for (int i = 0; i < VERB_BCF_COUNT; i++) dev_free(c->bc[i]);
     for (void* p : {(void*)c->Lf32, (void*)c->Uf32, (void*)c->lrhs, (void*)c->lres,
                     (void*)c->refine_red, (void*)c->trim_k0, (void*)c->trim_uoff,
                     (void*)c->maxabs_red})
-        cudaFree(p);
+        dev_free(p);
     free_krylov(c);
     free_kc(c);
     if (c->step_exec) cudaGraphExecDestroy(c->step_exec);
@@ -541,7 +663,7 @@ int verb_destroy(verb_ctx* c)
                     (void*)c->lwork, (void*)c->ipiv, (void*)c->conv_scratch,
                     (void*)c->conv_substeps, (void*)c->ticket, (void*)c->red, (void*)c->status,
                     (void*)c->Pa, (void*)c->kfwork, (void*)c->obs, (void*)c->kfticket})
-        cudaFree(p);
+        dev_free(p);
     for (int p = 0; p < PH_N; p++)
         for (EventPair& e : c->ev[p]) c->pool.push_back(e);
     for (EventPair& e : c->pool) {
@@ -648,7 +770,7 @@ int verb_upload_bc(verb_ctx* c, int b, const double* host)
 {
     if (!c || b < 0 || b >= VERB_BCF_COUNT || !host) return VERB_ERR_ARG;
     graph_invalidate(c);
-    if (!c->bc[b]) CK(cudaMalloc(&c->bc[b], bc_elems(c, b) * sizeof(double)));
+    if (!c->bc[b]) CK(dev_malloc((void**)&c->bc[b], bc_elems(c, b) * sizeof(double)));
     CK(cudaMemcpyAsync(c->bc[b], host, bc_elems(c, b) * sizeof(double), cudaMemcpyHostToDevice,
                        c->stream));
     return VERB_OK;
@@ -1112,9 +1234,35 @@ int verb_local_factor_lapack(verb_ctx* c, int p, int r, double* ab, long* ipiv1)
 // ====================================================== per-slice entry points
 namespace {
 
+// A per-slice call's block, for the calling thread
+struct ArenaUse {
+    Arena arena;
+    int take(size_t bytes)
+    {
+        const int s = arena_take(arena, bytes);
+        if (!s) t_arena = &arena;
+        return s;
+    }
+    ~ArenaUse()
+    {
+        t_arena = nullptr;
+        arena_put(arena);
+    }
+};
+
+// The context of one per-slice call
 struct TmpCtx {
+    ArenaUse use;  // outlives the context
     verb_ctx* c = nullptr;
-    ~TmpCtx() { verb_destroy(c); }
+    int open(int P, int R, int V, int K)
+    {
+        size_t bytes = 0;
+        if (int s = verb_estimate_device_bytes(P, R, V, K, VERB_PREC_FP64, 0, 0, &bytes)) return s;
+        // and what the estimate leaves out: alignment, the D_yx field, words
+        if (int s = use.take(bytes + 64 * 256 + sizeof(double) * (size_t)P * R * V * K)) return s;
+        return verb_create(&c, P, R, V, K, use.arena.stream);
+    }
+    ~TmpCtx() { verb_destroy(c); }  // drains the stream
 };
 
 }  // namespace
@@ -1125,8 +1273,10 @@ int verb_tridag(const double* a, const double* b, const double* c, const double*
                 long n)
 {
     if (!a || !b || !c || !r || !u || n < 1) return VERB_ERR_ARG;
+    ArenaUse use;
+    if (int s = use.take(sizeof(double) * 6 * n + 256)) return s;
     double* dv = nullptr;
-    CK(cudaMalloc(&dv, sizeof(double) * 6 * n));
+    CK(dev_malloc((void**)&dv, sizeof(double) * 6 * n));
     const double* src[4] = {a, b, c, r};
     int s = VERB_OK;
     for (int i = 0; i < 4 && !s; i++)
@@ -1135,7 +1285,7 @@ int verb_tridag(const double* a, const double* b, const double* c, const double*
         launch_tridag(dv, dv + n, dv + 2 * n, dv + 3 * n, dv + 4 * n, n, 0);
         s = cuda_ok(cudaMemcpy(u, dv + 4 * n, sizeof(double) * n, cudaMemcpyDeviceToHost));
     }
-    cudaFree(dv);
+    dev_free(dv);
     return s;
 }
 
@@ -1145,7 +1295,7 @@ int verb_diffusion_1d(double* psd, const double* x, int n, double lbc, double ub
 {
     if (!psd || !x || !D || !G || !S || !loss || n < 3) return VERB_ERR_ARG;
     TmpCtx t;
-    int s = verb_create(&t.c, 1, n, 1, 1, nullptr);
+    int s = t.open(1, n, 1, 1);
     if (s) return s;
     int types[VERB_BCF_COUNT] = {0, 0, 1, 1, lbc_t, ubc_t, 1, 1, 1, 1};
     if ((s = verb_set_bc_types(t.c, types))) return s;
@@ -1171,7 +1321,7 @@ int verb_diffusion_2d(double* psd, const double* x, const double* y, int nx, int
 {
     if (!psd || !x || !y || nx < 3 || ny < 3) return VERB_ERR_ARG;
     TmpCtx t;
-    int s = verb_create(&t.c, 1, 1, nx, ny, nullptr);
+    int s = t.open(1, 1, nx, ny);
     if (s) return s;
     int types[VERB_BCF_COUNT] = {0, 0, 1, 1, 1, 1, xl_t, xu_t, yl_t, yu_t};
     if ((s = verb_set_bc_types(t.c, types))) return s;
@@ -1183,8 +1333,8 @@ int verb_diffusion_2d(double* psd, const double* x, const double* y, int nx, int
         if ((s = verb_upload_field(t.c, fids[i], srcs[i]))) return s;
     const size_t n = (size_t)nx * ny;
     double* dkv = nullptr;
-    CK(cudaMalloc(&dkv, n * sizeof(double)));
-    s = cuda_ok(cudaMemcpy(dkv, Dyx, n * sizeof(double), cudaMemcpyHostToDevice));
+    CK(dev_malloc((void**)&dkv, n * sizeof(double)));
+    s = cuda_ok(cudaMemcpyAsync(dkv, Dyx, n * sizeof(double), cudaMemcpyHostToDevice, t.c->stream));
     t.c->dkv_override = dkv;
     if (!s) s = verb_upload_bc(t.c, VERB_BCF_VL, xl);
     if (!s) s = verb_upload_bc(t.c, VERB_BCF_VU, xu);
@@ -1208,9 +1358,13 @@ int verb_diffusion_2d(double* psd, const double* x, const double* y, int nx, int
                     L[j * klp + (i - 1)] = lu_cache[j * ldab + kv + i];
                 ip[j] = (int32_t)(index_cache[j] - 1);
             }
-            s = cuda_ok(cudaMemcpy(t.c->Lf, L.data(), L.size() * 8, cudaMemcpyHostToDevice));
-            if (!s) s = cuda_ok(cudaMemcpy(t.c->Uf, U.data(), U.size() * 8, cudaMemcpyHostToDevice));
-            if (!s) s = cuda_ok(cudaMemcpy(t.c->ipiv, ip.data(), n * 4, cudaMemcpyHostToDevice));
+            s = cuda_ok(cudaMemcpyAsync(t.c->Lf, L.data(), L.size() * 8, cudaMemcpyHostToDevice,
+                                                t.c->stream));
+            if (!s) s = cuda_ok(cudaMemcpyAsync(t.c->Uf, U.data(), U.size() * 8, cudaMemcpyHostToDevice,
+                                                t.c->stream));
+            if (!s) s = cuda_ok(cudaMemcpyAsync(t.c->ipiv, ip.data(), n * 4, cudaMemcpyHostToDevice,
+                                                t.c->stream));
+            if (!s) s = cuda_ok(cudaStreamSynchronize(t.c->stream));  // the host copies end here
             t.c->local_dirty = false;
             t.c->local_dt = dt / nsub;
         }
@@ -1219,7 +1373,7 @@ int verb_diffusion_2d(double* psd, const double* x, const double* y, int nx, int
     if (!s) s = verb_sync(t.c);
     if (!s) s = verb_download_psd(t.c, psd);
     if (!s && lu_cache && recompute_lu) s = verb_local_factor_lapack(t.c, 0, 0, lu_cache, index_cache);
-    cudaFree(dkv);
+    dev_free(dkv);
     return s;
 }
 
@@ -1230,8 +1384,10 @@ int verb_convection_1d(double* psd, const double* x, int n, double lbc, double u
     if ((lbc_t == VERB_BC_PERIODIC) != (ubc_t == VERB_BC_PERIODIC)) return VERB_ERR_BC;
     double* dv = nullptr;
     int* st = nullptr;
-    CK(cudaMalloc(&dv, sizeof(double) * 3 * n));
-    int s = cuda_ok(cudaMalloc(&st, sizeof(int)));
+    ArenaUse use;
+    if (int s = use.take(sizeof(double) * 3 * n + 512)) return s;
+    CK(dev_malloc((void**)&dv, sizeof(double) * 3 * n));
+    int s = cuda_ok(dev_malloc((void**)&st, sizeof(int)));
     if (!s) s = cuda_ok(cudaMemset(st, 0, sizeof(int)));
     if (!s) s = cuda_ok(cudaMemcpy(dv, psd, 8 * n, cudaMemcpyHostToDevice));
     if (!s) s = cuda_ok(cudaMemcpy(dv + n, x, 8 * n, cudaMemcpyHostToDevice));
@@ -1243,8 +1399,8 @@ int verb_convection_1d(double* psd, const double* x, int n, double lbc, double u
     int dst = 0;
     if (!s) s = cuda_ok(cudaMemcpy(psd, dv, 8 * n, cudaMemcpyDeviceToHost));
     if (!s) s = cuda_ok(cudaMemcpy(&dst, st, sizeof(int), cudaMemcpyDeviceToHost));
-    cudaFree(dv);
-    cudaFree(st);
+    dev_free(dv);
+    dev_free(st);
     return s ? s : dst;
 }
 
@@ -1255,7 +1411,7 @@ int verb_convection_2d(double* psd, const double* P, const double* R, int nP, in
 {
     if (!psd || !P || !R) return VERB_ERR_ARG;
     TmpCtx t;
-    int s = verb_create(&t.c, nP, nR, 1, 1, nullptr);
+    int s = t.open(nP, nR, 1, 1);
     if (s) return s;
     int types[VERB_BCF_COUNT] = {pl_t, pu_t, rl_t, ru_t, 1, 1, 1, 1, 1, 1};
     if ((s = verb_set_bc_types(t.c, types))) return s;
