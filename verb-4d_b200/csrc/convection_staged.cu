@@ -25,6 +25,7 @@
 // of many sub-steps takes as long as its lines are: 24 x 25 x 31 x 31 alone 9.9
 // ms, 2.7 here; 48 x 101 x 101 x 16 alone 47.4 ms, 23.2 here (one after the other
 // 31.0 -> 23.1 ms).
+#include "exact_div.cuh"
 #include "quickest.cuh"
 #include "verb_internal.cuh"
 
@@ -128,21 +129,6 @@ __device__ __forceinline__ void line_ghosts(double* E, int st, int n, int lt, in
 // the window is loaded once per group instead of shifted through registers.
 
 #ifdef VERB_BUILD_CONV_EXACT
-// a / b rounded to nearest with y = RN(1/b) (Markstein's correction, as in
-// div_const) for |a|, |b| in [2^-400, 2^400), where neither the quotient nor its
-// residual leaves the normal range; others are divided.
-__device__ __forceinline__ double div_by(double a, double b, double y)
-{
-    const double q = a * y;
-    const unsigned ea = ((unsigned)__double2hiint(a) & 0x7fffffffu) - 0x26f00000u;
-    const unsigned eb = ((unsigned)__double2hiint(b) & 0x7fffffffu) - 0x26f00000u;
-    if (eb < 0x32000000u) {
-        if (ea < 0x32000000u) return fma(fma(-q, b, a), y, q);
-        if (a == 0.0) return q;
-    }
-    return a / b;
-}
-
 // Unlimited values of U faces from the window d[k] = E[x-5+k], the roles of the
 // stencil's points chosen by the direction (QUICKEST6.cpp:169-186)
 template <int U>

@@ -253,18 +253,14 @@ int radial_run(verb_ctx* c, double dt)
     a.fbet = c->rfbet;
     a.fgam = c->rfgam;
     a.status = c->status;
-    if (c->radial_dirty || dt != c->radial_dt) {
-        PhaseTimer t(c, PH_RADF);
-        launch_radial_factor(a, c->stream);
-        c->acc.kernel_launches++;
-        c->radial_dirty = false;
-        c->radial_dt = dt;
-    }
+    const bool factor = c->radial_dirty || dt != c->radial_dt;
     {
-        PhaseTimer t(c, PH_RAD);
-        launch_radial_solve(a, c->stream);
+        PhaseTimer t(c, factor ? PH_RADF : PH_RAD);  // a step that factorises solves on the way
+        launch_radial_solve(a, factor, c->stream);
         c->acc.kernel_launches++;
     }
+    c->radial_dirty = false;
+    c->radial_dt = dt;
     return check_launch();
 }
 

@@ -39,6 +39,7 @@
 // -fmad=false) except the factorisation's rank-1 update, which both compute
 // as one fused multiply-add per element (fma()), so factors, pivots and
 // solutions are bit-identical to it.
+#include "exact_div.cuh"
 #include "verb_internal.cuh"
 
 #include <type_traits>
@@ -454,23 +455,6 @@ __device__ __forceinline__ void dmma(double2& c, double a, double b)
     asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
         : "+d"(c.x), "+d"(c.y)
         : "d"(a), "d"(b));
-}
-
-// RN(1 / x) for 2^-1000 < |x| < 2^1000: Newton steps from the hardware's
-// approximation, the last one correcting by the exact residual, which rounds
-// correctly except where the significand of x is all ones (Markstein, IBM J.
-// Res. Dev. 34, 1990); there 1/x lies just above the midpoint of a power of
-// two and its successor and rounds to the successor.  Without a division's
-// range branch the steps interleave with the pivot search.
-__device__ __forceinline__ double recip(double x)
-{
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-#pragma unroll
-    for (int i = 0; i < 4; i++) y = fma(y, fma(-x, y, 1.0), y);
-    const long long ones = 0xfffffffffffffLL;
-    const bool all = (__double_as_longlong(x) & ones) == ones;
-    return all ? __longlong_as_double(__double_as_longlong(y) | 1) : y;
 }
 
 // *p = (x, y) in shared memory where c holds, as a predicated store

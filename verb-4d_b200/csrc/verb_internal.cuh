@@ -43,8 +43,8 @@ struct RadialArgs {
     double *fa, *fbet, *fgam;  // cached Thomas factors [R][P*V*K]
     int* status;
 };
-void launch_radial_factor(const RadialArgs& a, cudaStream_t s);
-void launch_radial_solve(const RadialArgs& a, cudaStream_t s);
+// factor: forms the matrix and its cached recurrence on the way
+void launch_radial_solve(const RadialArgs& a, bool factor, cudaStream_t s);
 void launch_tridag(const double* a, const double* b, const double* c, const double* r, double* u,
                   long n, cudaStream_t s);
 
