@@ -490,9 +490,13 @@ def run_ours(args):
     if forms:
         out["forms"] = forms
     if world == 1 and rank == 0 and not args.no_cpu_baseline:
-        cb = reference_estimate(wl, budget_s=args.cpu_budget)
-        out["cpu_baseline"] = {"value": round(cb["value"], 8), "unit": "sim-hours/s",
-                               "cores": cb["cores"], "kind": "reference", "sample": cb["sample"]}
+        try:
+            cb = reference_estimate(wl, budget_s=args.cpu_budget)
+            out["cpu_baseline"] = {"value": round(cb["value"], 8), "unit": "sim-hours/s",
+                                   "cores": cb["cores"], "kind": "reference",
+                                   "sample": cb["sample"]}
+        except ReferenceMissing as e:
+            out["cpu_baseline"] = {"unavailable": str(e)}
     if rank == 0:
         print(json.dumps(out), flush=True)
     if world > 1:
@@ -738,6 +742,10 @@ def run_ensemble(args):
 
 
 # --------------------------------------------------------------------------- reference CPU path
+class ReferenceMissing(RuntimeError):
+    """The reference's sources or its compiled library are not on this machine."""
+
+
 class ReferenceSampler:
     """Times the reference's own routines (oracle/_ref, compiled from source) on
     bounded samples of one step of the workload and extrapolates to full steps.
@@ -759,7 +767,7 @@ class ReferenceSampler:
         if not O.have_reference():
             O.build(with_ref=None)
         if not O.have_reference():
-            raise RuntimeError("the reference library oracle/_ref is not built")
+            raise ReferenceMissing("the reference library oracle/_ref is not built")
         self.lib = O.reference(lu_caching=True).lib
         self.wl = wl
         self.cores = threads or len(os.sched_getaffinity(0))
@@ -893,7 +901,11 @@ def run_reference(args):
     hours = int(np.ceil((args.warmup + args.steps + 1) * W.DT_5MIN * 24)) + 1
     # the Kp series of the GPU arm (rank 0's seed): the same inputs hour by hour
     wl = W.make_workload(spec, seed=args.seed, kp=W.kp_series(args.seed, max(hours, 24)))
-    rs = ReferenceSampler(wl)
+    try:
+        rs = ReferenceSampler(wl)
+    except ReferenceMissing as e:
+        print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
+        return
     # each bench step is one bounded sample of a full step of the same hour
     # as the GPU arm's step; a few convection slices per step keeps the
     # whole --steps/--warmup run within minutes
