@@ -684,6 +684,18 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
 // (4.16); 48 x 51 x 45 x 21, 5 cells (and up to 512 threads) 23.5 (14.9) -> 13.9
 // (13.6); 48 x 101 x 61 x 13 40.7 (21.7) -> 24.4 (20.4).  With two slices on an SM
 // the slices of the most sub-steps slow each other: 24 x 51 alone 7.5 ms.
+//
+// That is for up to CG_WAVE slices an SM, where a pass waits for those slices.
+// Beyond, the slices there are decide: small ones take one more on an SM for each
+// CG_WAVE (24 x 25 x 47 x 31 4.19 (3.66) -> 3.97 (2.71) ms with two, 5.34 with one;
+// 24 x 25 x 61 x 61 9.03 (9.00) -> 6.58 (6.53) with three, 13.7 with one; 12 x 13 x
+// 61 x 61 2.47 (2.45) -> 1.57 (1.56)).  Where registers leave no room for three, the
+// line-job kernel is as fast or faster then and runs: 24 x 51 x 61 x 61 15.4 ms
+// against 22.9 with one slice on an SM, 24 x 51 x 47 x 31 6.83 (6.23) against 7.44
+// (6.03) with two; from 1800 points on only past 1.5 CG_WAVE: 36 x 76 x 47 x 31 20.9
+// (19.1) -> 18.8 (18.6), but 36 x 76 x 61 x 31 23.6 (23.6) against 24.1 (24.0), and
+// 48 x 101 x 61 x 61 94.8 against 95.6.  Slices below 400 points that come two an SM
+// or fewer are left to it too: 12 x 13 x 11 x 11 0.92 (0.35) against 1.05 (0.39).
 constexpr int CG_MAXT = 512;
 #ifdef VERB_BUILD_CONV_EXACT
 int cg_own(int P, int R)
@@ -691,10 +703,10 @@ int cg_own(int P, int R)
     const int n = P * R;
     return n < 400 ? 2 : (n >= 1000 && n < 1800 ? 8 : 5);
 }
-constexpr int CG_STEP = 3, CG_RESIDENT = 1;
+constexpr int CG_STEP = 3, CG_WAVE = 8;
 #else
 int cg_own(int P, int R) { return P * R < 1200 ? 5 : 11; }
-constexpr int CG_STEP = 6, CG_RESIDENT = 32;
+constexpr int CG_STEP = 6;
 #endif
 
 bool cg_shape(int P, int R, StagedShape& s)
@@ -724,12 +736,44 @@ StagedKernel cg_kernel(int P, int R, const StagedShape& s)
     return fn;
 }
 
+int cg_sms()
+{
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+// CTAs that an SM can hold
+int cg_resident(int P, int R)
+{
+    int per = 0;
+    StagedShape s;
+    if (!cg_shape(P, R, s)) return 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, cg_kernel(P, R, s), s.threads, cg_smem(P, R));
+    return std::max(per, 1);
+}
+
+// Whether this kernel is the faster one for so many slices (the contracted form
+// always is: 1.2 to 4 times from 12 x 13 to 48 x 101, 961 and 3721 slices)
+bool cg_faster(int P, int R, long long slices)
+{
+#ifdef VERB_BUILD_CONV_EXACT
+    const long long n = (long long)P * R, sms = cg_sms();
+    if (n < 400 && slices <= 2 * sms) return false;
+    if (2 * slices <= (n < 1800 ? 2 : 3) * CG_WAVE * sms) return true;
+    return n < 1000 && cg_resident(P, R) >= 3;
+#else
+    return true;
+#endif
+}
+
 }  // namespace
 }  // namespace VERB_STAGED_NS
 
 using namespace VERB_STAGED_NS;
 
-int VERB_STAGED(conv_staged_check)(int P, int R)
+int VERB_STAGED(conv_staged_check)(int P, int R, long long slices)
 {
     if (P < 11 || R < 11) return VERB_ERR_SIZE;
     int dev = 0, maxsm = 0;
@@ -737,21 +781,19 @@ int VERB_STAGED(conv_staged_check)(int P, int R)
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (cg_smem(P, R) > (size_t)maxsm || !cg_shape(P, R, s)) return VERB_ERR_SIZE;
-    return VERB_OK;
+    return cg_faster(P, R, slices) ? VERB_OK : VERB_ERR_SIZE;
 }
 
 size_t VERB_STAGED(conv_staged_scratch_doubles)(int P, int R) { return (cg_scratch(P, R) + 1) & ~(size_t)1; }
 
-int VERB_STAGED(conv_staged_ctas)(int P, int R)
+int VERB_STAGED(conv_staged_ctas)(int P, int R, long long slices)
 {
-    int dev = 0, sms = 0, per = 0;
-    StagedShape s;
-    if (!cg_shape(P, R, s)) return 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const StagedKernel fn = cg_kernel(P, R, s);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, s.threads, cg_smem(P, R));
-    return sms * std::min(std::max(per, 1), CG_RESIDENT);
+    const int sms = cg_sms();
+    long long per = cg_resident(P, R);
+#ifdef VERB_BUILD_CONV_EXACT
+    per = std::min(per, (slices + CG_WAVE * sms - 1) / (CG_WAVE * sms));
+#endif
+    return (int)std::min(sms * per, slices);
 }
 
 void VERB_STAGED(launch_convection_staged)(const ConvArgs& a, int nctas, cudaStream_t st)

@@ -442,14 +442,14 @@ int local_run(verb_ctx* c, double dt, double sub_dt)
 // every arithmetic mode, with no more CTAs than slices.
 size_t conv_scratch_size(const Dims& d)
 {
-    const size_t slices = (size_t)d.V * d.K;
-    auto ctas = [&](int n) { return std::min<size_t>(n, slices); };
+    const long long slices = (long long)d.V * d.K;
+    auto ctas = [&](int n) { return (size_t)std::min<long long>(n, slices); };
     const int P = d.P, R = d.R;
     size_t b = ctas(std::max(conv_ctas(P, R), conv_ctas_fma(P, R))) * conv_scratch_doubles(P, R);
-    if (conv_staged_check_exact(P, R) == VERB_OK)
-        b = std::max(b, ctas(conv_staged_ctas_exact(P, R)) * conv_staged_scratch_doubles_exact(P, R));
-    if (conv_staged_check(P, R) == VERB_OK)
-        b = std::max(b, ctas(conv_staged_ctas(P, R)) * conv_staged_scratch_doubles(P, R));
+    if (conv_staged_check_exact(P, R, slices) == VERB_OK)
+        b = std::max(b, conv_staged_ctas_exact(P, R, slices) * conv_staged_scratch_doubles_exact(P, R));
+    if (conv_staged_check(P, R, slices) == VERB_OK)
+        b = std::max(b, conv_staged_ctas(P, R, slices) * conv_staged_scratch_doubles(P, R));
     else if (conv_stream_check(P, R) == VERB_OK)
         b = std::max(b, ctas(conv_stream_ctas_max(P, R)) * conv_stream_scratch_doubles(P, R));
     return b * sizeof(double);
@@ -472,12 +472,13 @@ int conv_run(verb_ctx* c, double dt)
         int s = need_bc(c, b);
         if (s) return s;
     }
-    // the two-stage kernel where both sweeps run and a slice's planes fit the
-    // shared memory; other shapes take one thread per line (stream mode) or
-    // the line-job kernels of convection.cu
-    const bool staged = c->conv_arith == VERB_CONV_STREAM ? conv_staged_check(d.P, d.R) == VERB_OK
+    // the two-stage kernel where both sweeps run, a slice's planes fit the shared
+    // memory and it is the faster one (cg_faster); other shapes take one thread
+    // per line (stream mode) or the line-job kernels of convection.cu
+    const long long slices = (long long)d.V * d.K;
+    const bool staged = c->conv_arith == VERB_CONV_STREAM ? conv_staged_check(d.P, d.R, slices) == VERB_OK
                         : c->conv_arith == VERB_CONV_EXACT
-                            ? conv_staged_check_exact(d.P, d.R) == VERB_OK : false;
+                            ? conv_staged_check_exact(d.P, d.R, slices) == VERB_OK : false;
     const bool stream = c->conv_arith == VERB_CONV_STREAM && conv_stream_check(d.P, d.R) == VERB_OK;
     if (!stream)
         if (int s = (c->conv_arith == VERB_CONV_EXACT ? conv_check : conv_check_fma)(d.P, d.R)) return s;
@@ -516,9 +517,9 @@ int conv_run(verb_ctx* c, double dt)
     PhaseTimer t(c, PH_CONV);
     CK(cudaMemsetAsync(c->ticket, 0, sizeof(int), c->stream));
     if (staged && c->conv_arith == VERB_CONV_EXACT)
-        launch_convection_staged_exact(a, cap(conv_staged_ctas_exact(d.P, d.R)), c->stream);
+        launch_convection_staged_exact(a, conv_staged_ctas_exact(d.P, d.R, slices), c->stream);
     else if (staged)
-        launch_convection_staged(a, cap(conv_staged_ctas(d.P, d.R)), c->stream);
+        launch_convection_staged(a, conv_staged_ctas(d.P, d.R, slices), c->stream);
     else if (stream)
         launch_convection_stream(a, cap(conv_stream_ctas(d.P, d.R)), c->stream);
     else if (c->conv_arith == VERB_CONV_EXACT)

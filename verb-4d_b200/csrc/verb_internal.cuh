@@ -118,14 +118,14 @@ int conv_stream_ctas(int P, int R);
 int conv_stream_ctas_max(int P, int R);
 void launch_convection_stream(const ConvArgs& a, int nctas, cudaStream_t s);
 // two stages per pass over line segments (convection_staged.cu)
-int conv_staged_check(int P, int R);  // VERB_ERR_SIZE: the shape needs another kernel
+int conv_staged_check(int P, int R, long long slices);  // VERB_ERR_SIZE: another kernel's
 size_t conv_staged_scratch_doubles(int P, int R);
-int conv_staged_ctas(int P, int R);
+int conv_staged_ctas(int P, int R, long long slices);
 void launch_convection_staged(const ConvArgs& a, int nctas, cudaStream_t s);
 // the same in the reference's arithmetic (no contraction)
-int conv_staged_check_exact(int P, int R);
+int conv_staged_check_exact(int P, int R, long long slices);
 size_t conv_staged_scratch_doubles_exact(int P, int R);
-int conv_staged_ctas_exact(int P, int R);
+int conv_staged_ctas_exact(int P, int R, long long slices);
 void launch_convection_staged_exact(const ConvArgs& a, int nctas, cudaStream_t s);
 void launch_convection_line(double* psd, const double* x, int n, double lbc, double ubc, int lbc_t,
                             int ubc_t, const double* ux, double dt, int* status, cudaStream_t s);
