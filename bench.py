@@ -54,7 +54,7 @@ SOLVE_TRAFFIC_PER_ALG_BYTE = (9735437568 + 66170624) / 9698947584
 
 CONV_LABEL = {
     "fma": "fma: multiply-add contraction, within 1e-12 of the reference per step",
-    "stream": ("stream: one thread per line, all stages of a pass in registers, multiply-add "
+    "stream": ("stream: two stages over line segments, multiply-add "
                "contraction, within 1e-12 of the reference per step"),
     "exact": "exact: bit-identical to the reference",
 }
@@ -130,9 +130,9 @@ FP64_OPS_PER_FACE = 179
 # sm__inst_executed_pipe_fp64 over one launch at 48 x 101 x 101 x 8); the
 # op-count fraction above counts the reference's operations, the pipe share
 # the ones the kernel issues
-CONV_FP64_PIPE_NCU = {"fma": 0.336, "stream": 0.402, "exact": 0.471}
+CONV_FP64_PIPE_NCU = {"fma": 0.336, "stream": 0.337, "exact": 0.471}
 CONV_KERNEL = {"fma": "conv_fma::convection_kernel (nine warps per line job set)",
-               "stream": "convection_stream_kernel (one thread per line)",
+               "stream": "convection_staged_kernel (two stages over line segments)",
                "exact": "conv_exact::convection_kernel"}
 
 
@@ -953,7 +953,7 @@ def main():
                     help="replay steady-state steps from a captured CUDA graph (1) or launch "
                          "them eagerly with per-phase events (0)")
     ap.add_argument("--conv", default="stream", choices=["fma", "exact", "stream"],
-                    help="convection kernel: fma (contracted), stream (one thread per line, contracted) or exact (bit-identical)")
+                    help="convection kernel: fma (contracted), stream (contracted, two stages over line segments) or exact (bit-identical)")
     ap.add_argument("--trim", action="store_true",
                     help="ragged local systems: pitch angles outside the loss cone only")
     ap.add_argument("--ensemble", action="store_true", help="run the member ensemble instead")

@@ -266,14 +266,16 @@ int verb_autotune_local_solve(verb_ctx* ctx, double dt, double sub_dt, double* t
 /* Convection arithmetic.  VERB_CONV_EXACT (the default) restates the
  * reference's operations one by one without contraction, so results are
  * bit-identical to it (exp() of loss rates aside).  VERB_CONV_FMA runs the
- * same kernel compiled with multiply-add contraction (and nine warps per
- * block): about 18 % faster, and within a few units in the last place of the
- * exact form per step.  VERB_CONV_STREAM runs one thread per line through all
- * four stages of a pass at once (register windows, nothing staged between
- * stages), contracted, with the G product and the loss/source epilogue
- * applied as the sweeps store; it needs both sweeps (P and R >= 11) and
+ * line-job kernel compiled with multiply-add contraction, within a few units
+ * in the last place of the exact form per step.  VERB_CONV_STREAM is
+ * contracted too, with the G product and the loss/source epilogue applied as
+ * the sweeps store, and the fastest; it needs both sweeps (P and R >= 11) and
  * otherwise runs the VERB_CONV_FMA kernel; within a few units in the last
- * place of the reference per step.  Convection_2D
+ * place of the reference per step.  With both sweeps, VERB_CONV_EXACT and
+ * VERB_CONV_STREAM run the two-stage kernel over line segments where its three
+ * planes fit in shared memory (VERB_CONV_EXACT: and unless slices are so many
+ * that the line-job kernel is faster), else the line-job kernel and the kernel
+ * with one thread per line.  Convection_2D
  * (src/Convection_2D.cpp:36-169) has one arithmetic; the switch has no
  * counterpart in the reference. */
 #define VERB_CONV_EXACT 0

@@ -431,12 +431,12 @@ __device__ __forceinline__ void frw_wait_all() { asm volatile("cp.async.wait_all
 // skip is only taken where a panel holds a zero or tiny pivot or a value that
 // is not finite (the slow branches below).
 //
-// 24 x 51 x 101 x 21 (1224 systems, factors 12.9 GB): 55 ms for the unblocked
-// register-window kernel this replaces, 13.5 ms here; 24 x 25 x 31 x 31, the
-// mixed form's whole pass: 4.76 -> 1.98 ms.  The bound is the panel: about
-// 1000 cycles a column of pivot search and exchange through shared memory,
-// against 160-320 for the multiply-adds of the update, which run beside it,
-// and 4 of the 13.5 ms for writing the factors at the copy bandwidth.
+// 24 x 51 x 101 x 21 (1224 systems, factors 12.9 GB), the pass with the solve:
+// 60.5 ms with the unblocked register-window kernel this replaces, 16.1 ms here;
+// 24 x 25 x 31 x 31, the mixed form's pass: 4.76 -> 1.53 ms, 0.94 of it here.  The
+// bound is the panel: about 1000 cycles a column of pivot search and exchange
+// through shared memory, against 160-320 for the multiply-adds of the update,
+// which run beside it; writing the factors at the copy bandwidth takes 2 ms.
 constexpr int NB = 8;  // columns of a panel
 
 struct FBlk {
@@ -2006,10 +2006,11 @@ bool launch_factor_blk_t(const LocalArgs& a, cudaStream_t s)
     // the parking launch
     if (a.factors32 ? a.klp32 < 18 : a.klp < 9) return false;
     if (a.d.P * a.d.R > 65535) return false;
-    // PW: the kl + NB rows of a panel, one a thread.  Measured (GPU time of an
-    // upload-factorise-solve pass): 24 x 51 x 101 x 21 with 4 + 8 warps 18.9 ms
-    // (4 + 12: 19.3, 4 + 4: 22.9; panels of 16 columns 19.5-21.5);
-    // 24 x 25 x 31 x 31 with 2 + 2 warps 3.6 ms alone (2 + 4: 4.0; 16 columns 4.2).
+    // PW: the kl + NB rows of a panel, one a thread; the warps beside them share
+    // the update.  Measured while the kernel was built, an upload-factorise-solve
+    // pass: 24 x 51 x 101 x 21 with 4 + 8 warps 18.9 ms (4 + 12: 19.3, 4 + 4: 22.9;
+    // panels of 16 columns 19.5-21.5), 24 x 25 x 31 x 31 with 2 + 2 warps 3.6 ms
+    // alone (2 + 4: 4.0; 16 columns 4.2).
     const int kl = a.d.V + 1;
     if (kl + NB <= 32) launch_factor_blk<T, 1, 3>(a, s);
     else if (kl + NB <= 64) launch_factor_blk<T, 2, 4>(a, s);
