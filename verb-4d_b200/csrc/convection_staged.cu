@@ -97,7 +97,8 @@ struct Seg {
     int nl;
     const double *cr, *rc;  // c and 1 / |c| (0 for |c| <= 1e-31) of face k at [k * nl]
     // store epilogue of cell k: times e1 (P), or: times e1 plus e2 (R); the
-    // exact form divides by e3 (reciprocal e4) before, in the L sweep
+    // exact form divides by e3 (reciprocal e4) before, in the L sweep.  Where
+    // nothing is to be added it adds -0, which leaves a -0 as it is
     const double *e1, *e2, *e3, *e4;
 };
 
@@ -376,7 +377,7 @@ __device__ __forceinline__ void stage2(const Seg& L, double f0, bool last)
             c[u] = L.cr[at];
             rc[u] = L.rc[at];
             h1[u] = h3[u] = h4[u] = 1.0;
-            h2[u] = 0.0;
+            h2[u] = -0.0;
             at += L.nl;
             // cell x + u - 1 (the first group's entry of cell a - 1, and past
             // the table's ends, is not used)
@@ -467,7 +468,7 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
     double* crR = e1P + (size_t)PR;
     double* rcR = crR + (size_t)PR;
     double* e1R = rcR + (size_t)PR;            // exp(Loss dt)/G, or exp(Loss dt)
-    double* e2R = e1R + (size_t)PR;            // S dt, 0 at the ends
+    double* e2R = e1R + (size_t)PR;            // S dt, -0 at the ends
 #ifdef VERB_BUILD_CONV_EXACT
     double* e3R = e2R + (size_t)PR;            // G
     double* e4R = e3R + (size_t)PR;            // 1 / G
@@ -539,7 +540,7 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
 #else
             e1R[(size_t)iR * P + iP] = exp(a.loss[gi] * dtc) / G;
 #endif
-            e2R[(size_t)iR * P + iP] = iR && iR < R - 1 ? a.S[gi] * dtc : 0.0;
+            e2R[(size_t)iR * P + iP] = iR && iR < R - 1 ? a.S[gi] * dtc : -0.0;
         }
         // per-line CFL sub-cycles and face Courant numbers (QUICKEST6.cpp:37-52,
         // 150-160), one warp per line; velocity vel and grid x at (line, k)
