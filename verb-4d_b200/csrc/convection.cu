@@ -1066,10 +1066,7 @@ int conv_check_fma(int P, int R)
 {
     if ((P >= 3 && sweep_cfg(P, R - 1).lpl == 0) || (R >= 3 && sweep_cfg(R, P).lpl == 0))
         return VERB_ERR_SIZE;
-    int dev = 0, maxsm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (conv_smem_bytes_fma(P, R) > (size_t)maxsm) return VERB_ERR_SIZE;
+    if (conv_smem_bytes_fma(P, R) > allow_max_dynamic_smem((const void*)convection_kernel)) return VERB_ERR_SIZE;
     return VERB_OK;
 }
 
@@ -1105,10 +1102,7 @@ int conv_check(int P, int R)
 {
     if ((P >= 3 && sweep_cfg(P, R - 1).lpl == 0) || (R >= 3 && sweep_cfg(R, P).lpl == 0))
         return VERB_ERR_SIZE;
-    int dev = 0, maxsm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (conv_smem_bytes(P, R) > (size_t)maxsm) return VERB_ERR_SIZE;
+    if (conv_smem_bytes(P, R) > allow_max_dynamic_smem((const void*)convection_kernel)) return VERB_ERR_SIZE;
     return VERB_OK;
 }
 

@@ -777,11 +777,10 @@ using namespace VERB_STAGED_NS;
 int VERB_STAGED(conv_staged_check)(int P, int R, long long slices)
 {
     if (P < 11 || R < 11) return VERB_ERR_SIZE;
-    int dev = 0, maxsm = 0;
     StagedShape s;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (cg_smem(P, R) > (size_t)maxsm || !cg_shape(P, R, s)) return VERB_ERR_SIZE;
+    if (!cg_shape(P, R, s) ||
+        cg_smem(P, R) > allow_max_dynamic_smem((const void*)cg_kernel(P, R, s)))
+        return VERB_ERR_SIZE;
     return cg_faster(P, R, slices) ? VERB_OK : VERB_ERR_SIZE;
 }
 

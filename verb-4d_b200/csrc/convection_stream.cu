@@ -327,10 +327,8 @@ constexpr int CS_MINB = 3;
 int conv_stream_check(int P, int R)
 {
     if (P < 11 || R < 11) return VERB_ERR_SIZE;
-    int dev = 0, maxsm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (cs_smem(P, R) > (size_t)maxsm) return VERB_ERR_SIZE;
+    const auto fn = convection_stream_kernel<CS_U, CS_MINB>;
+    if (cs_smem(P, R) > allow_max_dynamic_smem((const void*)fn)) return VERB_ERR_SIZE;
     return VERB_OK;
 }
 

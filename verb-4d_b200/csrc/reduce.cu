@@ -6,29 +6,31 @@
 //  * max(PSD, 1e-21)        (src/VERB4D_Solver.cpp:621, 980, 1072, 1219)
 //  * field = base * scale   (UpdatableMatrix scale queue, src/UpdatableMatrix.cpp:698-708)
 // Grid-stride loops sized to a multiple of the SM count; one atomic per block.
+#include <map>
 #include <mutex>
-#include <set>
 #include <utility>
 
 #include "verb_internal.cuh"
 
 namespace verb {
 
-void allow_max_dynamic_smem(const void* func)
+size_t allow_max_dynamic_smem(const void* func)
 {
     static std::mutex mu;
-    static std::set<std::pair<const void*, int>> done;
+    static std::map<std::pair<const void*, int>, size_t> done;
     int dev = 0, maxsm = 0;
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lock(mu);
-    if (done.count({func, dev})) return;
+    const auto it = done.find({func, dev});
+    if (it != done.end()) return it->second;
     cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cudaFuncAttributes fa{};
-    if (cudaFuncGetAttributes(&fa, func) != cudaSuccess) return;
+    if (cudaFuncGetAttributes(&fa, func) != cudaSuccess) return 0;
     // the limit counts dynamic shared memory on top of the kernel's static part
     const int dyn = maxsm - (int)fa.sharedSizeBytes;
-    if (cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) == cudaSuccess)
-        done.insert({func, dev});
+    if (cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
+        return 0;
+    return done[{func, dev}] = (size_t)dyn;
 }
 
 namespace {
