@@ -85,7 +85,7 @@ int arena_take(Arena& a, size_t bytes)
     }
     a = Arena{};
     a.device = dev;
-    cudaError_t e = cudaMalloc(&a.base, bytes);
+    cudaError_t e = bytes ? cudaMalloc(&a.base, bytes) : cudaSuccess;
     if (e == cudaErrorMemoryAllocation && arenas_release()) {
         cudaGetLastError();
         e = cudaMalloc(&a.base, bytes);
@@ -101,10 +101,10 @@ int arena_take(Arena& a, size_t bytes)
 // the block's work is done
 void arena_put(Arena& a)
 {
-    if (!a.base) return;
+    if (!a.stream) return;
     Arena out = a;
     a = Arena{};
-    if (out.size <= ARENA_BYTES) {
+    if (out.base && out.size <= ARENA_BYTES) {
         std::lock_guard<std::mutex> lk(g_arena_mu);
         g_arenas.push_back(out);
         if (g_arenas.size() <= ARENA_KEEP) return;
@@ -283,10 +283,12 @@ int solve_variant_for(verb_ctx* c)
     return it == g_tuned_solve.end() ? -1 : it->second;  // -1: launch_local_solve's rule
 }
 
+constexpr int MAX_LOCAL_V = 111;  // solve windows hold kl+1 <= 128 and kv+1 <= 256
+
 int local_prepare(verb_ctx* c, LocalArgs& a, double dts)
 {
     const Dims& d = c->d;
-    if (d.V > 111) return VERB_ERR_ARG;  // solve windows hold kl+1 <= 128 and kv+1 <= 256
+    if (d.V > MAX_LOCAL_V) return VERB_ERR_ARG;
     for (int fid : {VERB_F_PSD, VERB_F_V, VERB_F_K, VERB_F_DVV, VERB_F_DKK, VERB_F_DVK,
                     VERB_F_G_LOCAL, VERB_F_LOSS_LOCAL, VERB_F_SOURCES}) {
         int s = need_field(c, fid);
@@ -1254,9 +1256,18 @@ struct TmpCtx {
     int open(int P, int R, int V, int K)
     {
         size_t bytes = 0;
-        if (int s = verb_estimate_device_bytes(P, R, V, K, VERB_PREC_FP64, 0, 0, &bytes)) return s;
+        // (no room for the factors of a band that the local phase refuses)
+        if (int s = verb_estimate_device_bytes(P, R, V, V > MAX_LOCAL_V ? 1 : K, VERB_PREC_FP64, 0, 0,
+                                               &bytes))
+            return s;
         // and what the estimate leaves out: alignment, the D_yx field, words
-        if (int s = use.take(bytes + 64 * 256 + sizeof(double) * (size_t)P * R * V * K)) return s;
+        int s = use.take(bytes + 64 * 256 + sizeof(double) * (size_t)P * R * V * K);
+        // the estimate covers every phase: a call may fit where its block does not
+        if (s == VERB_ERR_NOMEM) {
+            cudaGetLastError();
+            s = use.take(0);
+        }
+        if (s) return s;
         return verb_create(&c, P, R, V, K, use.arena.stream);
     }
     ~TmpCtx() { verb_destroy(c); }  // drains the stream
