@@ -22,69 +22,102 @@ size_t bc_elems(const verb_ctx* c, int b)
 // stream 0.1 ms, the kernels of a 24 x 25 convection slice 0.07 ms), so up to
 // ARENA_KEEP blocks of up to ARENA_BYTES each are kept idle between calls.  A
 // block serves one call at a time (taken and put back under the lock, its
-// stream drained before); idle blocks are given back when an allocation fails
-// and at exit.  What a block has no room for is allocated by itself.
+// stream drained before); idle blocks are given back when dev_malloc finds no
+// memory and at exit.  What a block has no room for is allocated by itself.
+//
+// A block belongs to the CUDA context it was made in (its handle and its id: a
+// device reset makes a new context with the old handle, in which an old address
+// may be someone else's memory).  It is used and freed in that context only, and
+// forgotten once a new one has the handle.
 struct Arena {
     char* base = nullptr;
     size_t size = 0, used = 0;
     int device = -1;
+    CUcontext ctx = nullptr;
+    unsigned long long id = 0;  // 0: not known
     cudaStream_t stream = nullptr;
 };
-constexpr size_t ARENA_KEEP = 4, ARENA_BYTES = (size_t)16 << 20;
+constexpr int ARENA_KEEP = 4;     // of one context
+constexpr int ARENA_SLOTS = 32;   // of all
+constexpr size_t ARENA_BYTES = (size_t)16 << 20;
 std::mutex g_arena_mu;
-std::vector<Arena> g_arenas;          // idle
+Arena g_arenas[ARENA_SLOTS];  // idle ones have a base
 thread_local Arena* t_arena = nullptr;  // of the call this thread is in
 
+// the calling thread's CUDA context; make: also where it has none yet
+void current_context(CUcontext& ctx, unsigned long long& id, bool make)
+{
+    typedef CUresult (*GetCurrent)(CUcontext*);
+    typedef CUresult (*GetId)(CUcontext, unsigned long long*);
+    static const auto entry = [](const char* name) {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPoint(name, &fn, cudaEnableDefault, &r) != cudaSuccess ||
+            r != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            fn = nullptr;
+        }
+        return fn;
+    };
+    static const GetCurrent get_current = (GetCurrent)entry("cuCtxGetCurrent");
+    static const GetId get_id = (GetId)entry("cuCtxGetId");
+    ctx = nullptr;
+    id = 0;
+    if (!get_current || !get_id) return;
+    for (int turn = 0;; turn++) {
+        if (get_current(&ctx) == CUDA_SUCCESS && ctx && get_id(ctx, &id) == CUDA_SUCCESS) return;
+        id = 0;
+        if (turn > 0 || !make || cudaFree(nullptr) != cudaSuccess) return;
+    }
+}
+
+// in the calling thread's context, which is the block's
 void arena_free(Arena& a)
 {
-    int dev = -1;
-    cudaGetDevice(&dev);
-    if (a.device >= 0 && a.device != dev) cudaSetDevice(a.device);
     if (a.stream) cudaStreamDestroy(a.stream);
     cudaFree(a.base);
-    if (a.device >= 0 && a.device != dev) cudaSetDevice(dev);
     a = Arena{};
 }
 
-// idle blocks back to the device; true when there were any
+// idle blocks of the calling thread's context back to it; true when there were any
 bool arenas_release()
 {
-    std::vector<Arena> idle;
+    CUcontext ctx;
+    unsigned long long id;
+    current_context(ctx, id, false);
+    Arena idle[ARENA_SLOTS];
+    int n = 0;
     {
         std::lock_guard<std::mutex> lk(g_arena_mu);
-        idle.swap(g_arenas);
+        for (Arena& a : g_arenas)
+            if (a.base && id && a.ctx == ctx && a.id == id) {
+                idle[n++] = a;
+                a = Arena{};
+            }
     }
-    for (Arena& a : idle) arena_free(a);
-    return !idle.empty();
+    for (int i = 0; i < n; i++) arena_free(idle[i]);
+    return n > 0;
 }
 
 int arena_take(Arena& a, size_t bytes)
 {
-    int dev = 0;
-    CK(cudaGetDevice(&dev));
-    Arena got;
+    a = Arena{};
+    CK(cudaGetDevice(&a.device));
+    current_context(a.ctx, a.id, true);
     {
         std::lock_guard<std::mutex> lk(g_arena_mu);
-        for (size_t i = g_arenas.size(); i-- > 0;)
-            if (g_arenas[i].device == dev && g_arenas[i].size >= bytes) {
-                got = g_arenas[i];
-                g_arenas.erase(g_arenas.begin() + i);
-                break;
-            }
-    }
-    if (got.base) {
-        // still there (the device may have been reset in between)
-        cudaPointerAttributes at{};
-        if (cudaPointerGetAttributes(&at, got.base) == cudaSuccess &&
-            at.type == cudaMemoryTypeDevice && cudaStreamQuery(got.stream) == cudaSuccess) {
-            a = got;
+        Arena* fit = nullptr;  // the smallest that is large enough
+        for (Arena& g : g_arenas)
+            if (g.base && a.id && g.ctx == a.ctx && g.id == a.id && g.size >= bytes &&
+                (!fit || g.size < fit->size))
+                fit = &g;
+        if (fit) {
+            a = *fit;
+            *fit = Arena{};
             a.used = 0;
             return VERB_OK;
         }
-        cudaGetLastError();
     }
-    a = Arena{};
-    a.device = dev;
     cudaError_t e = bytes ? cudaMalloc(&a.base, bytes) : cudaSuccess;
     if (e == cudaErrorMemoryAllocation && arenas_release()) {
         cudaGetLastError();
@@ -104,12 +137,25 @@ void arena_put(Arena& a)
     if (!a.stream) return;
     Arena out = a;
     a = Arena{};
-    if (out.base && out.size <= ARENA_BYTES) {
+    if (out.base && out.size <= ARENA_BYTES && out.id) {
         std::lock_guard<std::mutex> lk(g_arena_mu);
-        g_arenas.push_back(out);
-        if (g_arenas.size() <= ARENA_KEEP) return;
-        out = g_arenas.front();
-        g_arenas.erase(g_arenas.begin());
+        int own = 0, at = -1, smallest = -1;
+        for (int i = 0; i < ARENA_SLOTS; i++) {
+            Arena& g = g_arenas[i];
+            if (g.base && g.ctx == out.ctx && g.id != out.id) g = Arena{};  // gone with its context
+            if (!g.base) {
+                at = i;
+            } else if (g.ctx == out.ctx) {
+                own++;
+                if (smallest < 0 || g.size < g_arenas[smallest].size) smallest = i;
+            }
+        }
+        if (own < ARENA_KEEP && at >= 0) {
+            g_arenas[at] = out;
+            return;
+        }
+        // the larger blocks are kept: they serve more calls
+        if (smallest >= 0 && g_arenas[smallest].size < out.size) std::swap(g_arenas[smallest], out);
     }
     arena_free(out);
 }

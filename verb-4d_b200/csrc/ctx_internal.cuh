@@ -4,6 +4,7 @@
 // assimilation).  Private to the library.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cmath>
