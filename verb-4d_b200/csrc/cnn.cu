@@ -316,14 +316,14 @@ extern "C" int verb_cnn_create(verb_cnn** out, int layers, const int* channels, 
         n->amax = std::max(n->amax, (size_t)max_batch * std::max(channels[l], channels[l + 1]) * HW);
     }
     n->np = off;
-    int s = ck(cudaMalloc(&n->p, off * sizeof(float)));
-    if (!s) s = ck(cudaMalloc(&n->g, off * sizeof(float)));
-    if (!s) s = ck(cudaMalloc(&n->m, off * sizeof(float)));
-    if (!s) s = ck(cudaMalloc(&n->v, off * sizeof(float)));
-    if (!s) s = ck(cudaMalloc(&n->ph, off * sizeof(__half)));
-    if (!s) s = ck(cudaMalloc(&n->act, aoff * sizeof(float)));
-    if (!s) s = ck(cudaMalloc(&n->grad, 2 * n->amax * sizeof(float)));
-    if (!s) s = ck(cudaMalloc(&n->loss, sizeof(float)));
+    int s = ck(vctx::dev_malloc((void**)&n->p, off * sizeof(float)));
+    if (!s) s = ck(vctx::dev_malloc((void**)&n->g, off * sizeof(float)));
+    if (!s) s = ck(vctx::dev_malloc((void**)&n->m, off * sizeof(float)));
+    if (!s) s = ck(vctx::dev_malloc((void**)&n->v, off * sizeof(float)));
+    if (!s) s = ck(vctx::dev_malloc((void**)&n->ph, off * sizeof(__half)));
+    if (!s) s = ck(vctx::dev_malloc((void**)&n->act, aoff * sizeof(float)));
+    if (!s) s = ck(vctx::dev_malloc((void**)&n->grad, 2 * n->amax * sizeof(float)));
+    if (!s) s = ck(vctx::dev_malloc((void**)&n->loss, sizeof(float)));
     if (!s) s = ck(cudaMemsetAsync(n->m, 0, off * sizeof(float), n->s));
     if (!s) s = ck(cudaMemsetAsync(n->v, 0, off * sizeof(float), n->s));
     if (s) {
@@ -339,7 +339,7 @@ extern "C" int verb_cnn_destroy(verb_cnn* n)
     if (!n) return VERB_OK;
     for (void* q : {(void*)n->p, (void*)n->g, (void*)n->m, (void*)n->v, (void*)n->ph, (void*)n->act,
                     (void*)n->grad, (void*)n->loss})
-        cudaFree(q);
+        vctx::dev_free(q);
     delete n;
     return VERB_OK;
 }

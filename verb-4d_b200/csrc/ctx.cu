@@ -22,8 +22,8 @@ size_t bc_elems(const verb_ctx* c, int b)
 // stream 0.1 ms, the kernels of a 24 x 25 convection slice 0.07 ms), so up to
 // ARENA_KEEP blocks of up to ARENA_BYTES each are kept idle between calls.  A
 // block serves one call at a time (taken and put back under the lock, its
-// stream drained before); idle blocks are given back when dev_malloc finds no
-// memory and at exit.  What a block has no room for is allocated by itself.
+// stream drained before); idle blocks are given back when an allocation of this
+// library finds no memory (dev_malloc) and at exit.  What a block has no room for is allocated by itself.
 //
 // A block belongs to the CUDA context it was made in (its handle and its id: a
 // device reset makes a new context with the old handle, in which an old address
@@ -768,7 +768,7 @@ static int upload_common(verb_ctx* c, int fid, const void* src, cudaMemcpyKind k
     } else {
         CK(cudaMemcpyAsync(c->f[fid], src, bytes, kind, c->stream));
         if (c->fbase[fid]) {
-            cudaFree(c->fbase[fid]);
+            dev_free(c->fbase[fid]);
             c->fbase[fid] = nullptr;
         }
     }
@@ -796,7 +796,7 @@ int verb_set_field_scale(verb_ctx* c, int fid, double scale)
     if (c->f[fid]) {
         if (!c->fbase[fid]) {
             // the current contents are the base (scale 1) field
-            CK(cudaMalloc(&c->fbase[fid], bytes));
+            CK(dev_malloc((void**)&c->fbase[fid], bytes));
             CK(cudaMemcpyAsync(c->fbase[fid], c->f[fid], bytes, cudaMemcpyDeviceToDevice, c->stream));
         }
         if (scale != 1.0) {
@@ -861,12 +861,12 @@ int verb_set_local_precision(verb_ctx* c, int mode, int refinements)
         // allocates this one's
         CK(cudaStreamSynchronize(c->stream));
         if (mode == VERB_PREC_MIXED) {
-            cudaFree(c->Lf);
-            cudaFree(c->Uf);
+            dev_free(c->Lf);
+            dev_free(c->Uf);
             c->Lf = c->Uf = nullptr;
         } else {
-            cudaFree(c->Lf32);
-            cudaFree(c->Uf32);
+            dev_free(c->Lf32);
+            dev_free(c->Uf32);
             c->Lf32 = c->Uf32 = nullptr;
         }
         c->local_prec = mode;
@@ -989,7 +989,7 @@ int verb_autotune_local_solve(verb_ctx* c, double dt, double sub_dt, double* tim
     const size_t nu = c->local_unknowns;
     launch_local_rhs(a, false, c->stream);
     double* keep = nullptr;
-    CK(cudaMalloc(&keep, nu * sizeof(double)));
+    CK(dev_malloc((void**)&keep, nu * sizeof(double)));
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -1021,7 +1021,7 @@ int verb_autotune_local_solve(verb_ctx* c, double dt, double sub_dt, double* tim
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    cudaFree(keep);
+    dev_free(keep);
     if (st) return st;
     c->solve_variant = best;
     {
@@ -1503,7 +1503,7 @@ int verb_assimilate_radial(verb_ctx* c, const double* obs_host, double dt, doubl
     if (c->Pa && p_index != c->pa_p_index) return VERB_ERR_ARG;
     const size_t cols = (size_t)(p_index >= 0 ? 1 : d.P) * d.V * d.K, RR = (size_t)d.R * d.R;
     if (!c->Pa) {
-        CK(cudaMalloc(&c->Pa, cols * RR * sizeof(double)));
+        CK(dev_malloc((void**)&c->Pa, cols * RR * sizeof(double)));
         CK(cudaMemsetAsync(c->Pa, 0, cols * RR * sizeof(double), c->stream));
         c->pa_p_index = p_index;
     }
@@ -1534,9 +1534,9 @@ int verb_assimilate_radial(verb_ctx* c, const double* obs_host, double dt, doubl
     const int nctas = kf_ctas(d, p_index);
     const size_t wb = (size_t)nctas * kf_work_doubles(d.R) * sizeof(double);
     if (wb > c->kfwork_bytes) {
-        cudaFree(c->kfwork);
+        dev_free(c->kfwork);
         c->kfwork = nullptr;
-        CK(cudaMalloc(&c->kfwork, wb));
+        CK(dev_malloc((void**)&c->kfwork, wb));
         c->kfwork_bytes = wb;
     }
     CK(alloc((void**)&c->kfticket, sizeof(int)));
@@ -1578,7 +1578,7 @@ bool pop_component(UpdComponent& k, double t, double** new_base)
     double* data = nullptr;
     double data_time = 0;
     while (!k.data_q.empty() && t >= k.data_q.front().first) {
-        if (data) cudaFree(data);  // superseded before it was used
+        if (data) dev_free(data);  // superseded before it was used
         data = k.data_q.front().second;
         data_time = k.data_q.front().first;
         k.data_q.pop_front();
@@ -1589,7 +1589,7 @@ bool pop_component(UpdComponent& k, double t, double** new_base)
             k.last_update_time = t;
             updated = true;
         } else {
-            cudaFree(data);
+            dev_free(data);
         }
     }
     // scale (:676-695) and limits (:724-788): the latest due value, updated
@@ -1620,7 +1620,7 @@ int verb_field_add_component(verb_ctx* c, int fid, const double* host_base, int*
     UpdField& u = *c->upd[fid];
     if ((int)u.comps.size() >= MAX_COMPONENTS) return VERB_ERR_SIZE;
     UpdComponent k;
-    CK(cudaMalloc(&k.base, npts(c) * sizeof(double)));
+    CK(dev_malloc((void**)&k.base, npts(c) * sizeof(double)));
     CK(cudaMemcpyAsync(k.base, host_base, npts(c) * sizeof(double), cudaMemcpyHostToDevice,
                        c->stream));
     u.comps.push_back(k);
@@ -1646,7 +1646,7 @@ int verb_component_queue_data(verb_ctx* c, int fid, int comp, double time, const
     if (int s = component_of(c, fid, comp, &k)) return s;
     if (!host || (!k->data_q.empty() && time < k->data_q.back().first)) return VERB_ERR_ARG;
     double* d = nullptr;
-    CK(cudaMalloc(&d, npts(c) * sizeof(double)));
+    CK(dev_malloc((void**)&d, npts(c) * sizeof(double)));
     CK(cudaMemcpyAsync(d, host, npts(c) * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     k->data_q.emplace_back(time, d);
     return VERB_OK;
@@ -1690,7 +1690,7 @@ int verb_update_fields(verb_ctx* c, double current_time, unsigned int* updated_m
                 double* old = k.base;
                 k.base = nb;
                 CK(cudaStreamSynchronize(c->stream));
-                cudaFree(old);
+                dev_free(old);
             }
         }
         if (!changed) continue;
@@ -1761,7 +1761,7 @@ int verb_write_field_pltb(verb_ctx* c, int fid, const char* path, int async_writ
     if (int s = verb_output_wait(c)) return s;
     const size_t bytes = npts(c) * sizeof(double);
     if (!c->out_snap) {
-        CK(cudaMalloc(&c->out_snap, bytes));
+        CK(dev_malloc((void**)&c->out_snap, bytes));
         CK(cudaMallocHost(&c->out_host, bytes));
         CK(cudaStreamCreateWithFlags(&c->out_stream, cudaStreamNonBlocking));
         CK(cudaEventCreateWithFlags(&c->out_ev_snap, cudaEventDisableTiming));
@@ -1830,8 +1830,8 @@ int verb_remap_L(verb_ctx* c, const double* new_L_host)
     if (c->upd[VERB_F_L]) return VERB_ERR_ARG;
     const size_t bytes = npts(c) * sizeof(double);
     double *newL = nullptr, *scratch = nullptr;
-    CK(cudaMalloc(&newL, bytes));
-    int s = cuda_ok(cudaMalloc(&scratch, 2 * bytes));
+    CK(dev_malloc((void**)&newL, bytes));
+    int s = cuda_ok(dev_malloc((void**)&scratch, 2 * bytes));
     if (!s) s = cuda_ok(cudaMemcpyAsync(newL, new_L_host, bytes, cudaMemcpyHostToDevice, c->stream));
     if (!s) {
         launch_remap(c->f[VERB_F_PSD], c->f[VERB_F_L], newL, scratch, scratch + npts(c), c->d,
@@ -1841,8 +1841,8 @@ int verb_remap_L(verb_ctx* c, const double* new_L_host)
     }
     if (!s) s = cuda_ok(cudaMemcpyAsync(c->f[VERB_F_L], newL, bytes, cudaMemcpyDeviceToDevice, c->stream));
     if (!s) s = cuda_ok(cudaStreamSynchronize(c->stream));
-    cudaFree(newL);
-    cudaFree(scratch);
+    dev_free(newL);
+    dev_free(scratch);
     if (s) return s;
     mark_dirty(c, VERB_F_L);
     return verb_sync(c);
@@ -1897,12 +1897,12 @@ int verb_set_local_trim(verb_ctx* c, const int* k0_host)
     // the factor arrays change size: release them (refactored at the next solve)
     for (void** p : {(void**)&c->Lf, (void**)&c->Uf, (void**)&c->Lf32, (void**)&c->Uf32,
                      (void**)&c->ipiv, (void**)&c->lwork, (void**)&c->lrhs, (void**)&c->lres}) {
-        cudaFree(*p);
+        dev_free(*p);
         *p = nullptr;
     }
     free_krylov(c);
-    cudaFree(c->trim_k0);
-    cudaFree(c->trim_uoff);
+    dev_free(c->trim_k0);
+    dev_free(c->trim_uoff);
     c->trim_k0 = nullptr;
     c->trim_uoff = nullptr;
     c->local_dirty = true;
@@ -1917,8 +1917,8 @@ int verb_set_local_trim(verb_ctx* c, const int* k0_host)
         off[s] = tot;
         tot += (long long)d.V * (d.K - k0_host[s]);
     }
-    CK(cudaMalloc(&c->trim_k0, nsys * sizeof(int)));
-    CK(cudaMalloc(&c->trim_uoff, nsys * sizeof(long long)));
+    CK(dev_malloc((void**)&c->trim_k0, nsys * sizeof(int)));
+    CK(dev_malloc((void**)&c->trim_uoff, nsys * sizeof(long long)));
     CK(cudaMemcpy(c->trim_k0, k0_host, nsys * sizeof(int), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c->trim_uoff, off.data(), nsys * sizeof(long long), cudaMemcpyHostToDevice));
     c->local_unknowns = (size_t)tot;

@@ -11,7 +11,7 @@ void free_kc(verb_ctx* c)
     for (void** p : {(void**)&c->kc_M, (void**)&c->kc_Pa, (void**)&c->kc_W, (void**)&c->kc_vec,
                      (void**)&c->kc_int})
     {
-        cudaFree(*p);
+        dev_free(*p);
         *p = nullptr;
     }
     c->kc_valid = false;
@@ -94,7 +94,7 @@ int kc_run(verb_ctx* c, const double* obs_host, double dt, double model_error, d
     B = std::min(B, nsl);
     if (c->kc_chunk != B) {
         for (void** p : {(void**)&c->kc_W, (void**)&c->kc_vec, (void**)&c->kc_int}) {
-            cudaFree(*p);
+            dev_free(*p);
             *p = nullptr;
         }
         c->kc_chunk = B;

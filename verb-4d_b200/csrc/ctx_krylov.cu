@@ -13,7 +13,7 @@ void free_krylov(verb_ctx* c)
                      (void**)&c->kscale, (void**)&c->kiters, (void**)&c->kpend,
                      (void**)&c->kcount, (void**)&c->kmax, (void**)&c->kprev,
                      (void**)&c->kpfeat, (void**)&c->kpc}) {
-        cudaFree(*p);
+        dev_free(*p);
         *p = nullptr;
     }
 }

@@ -7,6 +7,13 @@
 
 #include "verb4d_b200.h"
 
+namespace vctx {
+// cudaMalloc and cudaFree of the library: with the block of a per-slice call
+// that the thread is in, and idle blocks given back where memory has run out
+cudaError_t dev_malloc(void** p, size_t bytes);
+void dev_free(void* p);
+}  // namespace vctx
+
 namespace verb {
 
 // Raise a kernel's dynamic shared-memory limit to the device maximum, once per
