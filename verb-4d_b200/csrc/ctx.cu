@@ -1339,6 +1339,7 @@ int verb_tridag(const double* a, const double* b, const double* c, const double*
         launch_tridag(dv, dv + n, dv + 2 * n, dv + 3 * n, dv + 4 * n, n, 0);
         s = cuda_ok(cudaMemcpy(u, dv + 4 * n, sizeof(double) * n, cudaMemcpyDeviceToHost));
     }
+    if (s) cudaStreamSynchronize(0);  // the block's next call has a stream of its own
     dev_free(dv);
     return s;
 }
@@ -1453,6 +1454,7 @@ int verb_convection_1d(double* psd, const double* x, int n, double lbc, double u
     int dst = 0;
     if (!s) s = cuda_ok(cudaMemcpy(psd, dv, 8 * n, cudaMemcpyDeviceToHost));
     if (!s) s = cuda_ok(cudaMemcpy(&dst, st, sizeof(int), cudaMemcpyDeviceToHost));
+    if (s) cudaStreamSynchronize(0);  // the block's next call has a stream of its own
     dev_free(dv);
     dev_free(st);
     return s ? s : dst;
