@@ -84,7 +84,10 @@ typedef enum {
 typedef struct verb_ctx verb_ctx;
 
 /* Phase timings (milliseconds, CUDA events on the context stream), filled when
- * timing is enabled with verb_set_timing(ctx, 1). */
+ * timing is enabled with verb_set_timing(ctx, 1).  A radial pass whose matrix
+ * changed forms it and its recurrence on the way: such a pass is wholly in
+ * radial_factor_ms, the others in radial_ms.  local_ms covers the local phase,
+ * local_factor_ms and local_solve_ms its parts. */
 typedef struct {
     double convection_ms, radial_ms, radial_factor_ms, local_ms, local_factor_ms,
         local_solve_ms, reduce_ms, kf_ms;

@@ -314,6 +314,10 @@ class Context:
         L.check(self.lib.verb_set_timing(self.h, 1 if on else 0), "timing")
 
     def timing(self) -> dict:
+        """Phase times in ms since timing was enabled.  A radial pass whose
+        matrix changed is wholly in radial_factor_ms (it solves on the way),
+        the others in radial_ms; local_ms includes local_factor_ms and
+        local_solve_ms."""
         t = L.Timing()
         L.check(self.lib.verb_get_timing(self.h, C.byref(t)), "timing")
         return {n: getattr(t, n) for n, _ in L.Timing._fields_}
