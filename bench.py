@@ -54,8 +54,8 @@ SOLVE_TRAFFIC_PER_ALG_BYTE = (9735437568 + 66170624) / 9698947584
 
 CONV_LABEL = {
     "fma": "fma: multiply-add contraction, within 1e-12 of the reference per step",
-    "stream": ("stream: two stages over line segments, multiply-add "
-               "contraction, within 1e-12 of the reference per step"),
+    "stream": ("stream: multiply-add contraction, store epilogues in the sweeps, "
+               "within 1e-12 of the reference per step"),
     "exact": "exact: bit-identical to the reference",
 }
 
@@ -126,14 +126,25 @@ class ClockSampler:
 
 
 FP64_OPS_PER_FACE = 179
-# FP64-pipe share of each convection kernel's active cycles (ncu
-# sm__inst_executed_pipe_fp64 over one launch at 48 x 101 x 101 x 8); the
-# op-count fraction above counts the reference's operations, the pipe share
-# the ones the kernel issues
-CONV_FP64_PIPE_NCU = {"fma": 0.336, "stream": 0.337, "exact": 0.471}
-CONV_KERNEL = {"fma": "conv_fma::convection_kernel (nine warps per line job set)",
-               "stream": "convection_staged_kernel (two stages over line segments)",
-               "exact": "conv_exact::convection_kernel"}
+# The kernel of a convection pass by arithmetic and dispatch
+# (Context.convection_kernel), and its FP64-pipe share of active cycles where it
+# was profiled: slices of 48 x 101 (ncu sm__inst_executed_pipe_fp64 over one
+# launch at 48 x 101 x 101 x 8).  The op-count fraction below counts the
+# reference's operations, the pipe share the ones the kernel issues
+CONV_KERNEL = {("fma", "lines"): ("conv_fma::convection_kernel (nine warps per line job set)", 0.336),
+               ("stream", "lines"): ("conv_fma::convection_kernel (nine warps per line job set)", 0.336),
+               ("stream", "staged"): ("convection_staged_kernel (two stages over line segments)", 0.337),
+               ("stream", "stream"): ("convection_stream_kernel (one thread per line)", 0.402),
+               ("exact", "lines"): ("conv_exact::convection_kernel (eight warps per line job set)", 0.471),
+               ("exact", "staged"): ("conv_staged_exact::convection_staged_kernel (two stages over "
+                                     "line segments)", 0.489)}
+
+
+def conv_kernel_entry(arith, kernel, P, R):
+    """Name and profiled FP64-pipe share (None where slices of this shape were
+    not profiled) of the convection kernel that ran."""
+    name, pipe = CONV_KERNEL[arith, kernel]
+    return name, pipe if (P, R) == (48, 101) else None
 
 
 def fp64_peak_tops():
@@ -268,6 +279,7 @@ def run_ours(args):
     neg = ctx.negative_count()
     dev_bytes = ctx.device_bytes()
     conv_substeps = int(ctx.convection_substeps().astype(np.int64).sum())
+    conv_name, conv_pipe = conv_kernel_entry(args.conv, ctx.convection_kernel(), *spec.shape[:2])
     form_info = None
     if args.form == "mixed":
         # the same steps in the FP64 form, for the error of the mixed form and
@@ -467,15 +479,16 @@ def run_ours(args):
                                         else "algorithmic bytes x 1.0106, the DRAM/algorithmic "
                                              "ratio of one ncu-captured launch at 48x101x101x8 "
                                              "(the 48x101x101x91 band, kl = 102)")},
-        "roofline_fp64": {"kernel": CONV_KERNEL[args.conv] + ", ULTIMATE-QUICKEST sweeps, FP64",
+        "roofline_fp64": {"kernel": conv_name + ", ULTIMATE-QUICKEST sweeps, FP64",
                           "bound": "fp64", "achieved": round(conv_tops, 3), "peak": fp64_peak,
                           "unit": "TOP/s", "frac": round(conv_tops / fp64_peak, 4),
                           "peak_source": "nominal FP64 issue rate, 148 SMs x 64 lanes at "
                                          "MEASURED_PEAKS.json sm_max_mhz",
                           "fp64_ops_per_face": FP64_OPS_PER_FACE,
-                          "fp64_pipe_active_ncu": CONV_FP64_PIPE_NCU[args.conv],
-                          "fp64_pipe_source": "ncu inst_executed_pipe_fp64 over active cycles, "
-                                              "one launch of this kernel at 48x101x101x8",
+                          "fp64_pipe_active_ncu": conv_pipe,
+                          "fp64_pipe_source": ("ncu inst_executed_pipe_fp64 over active cycles, "
+                                               "one launch of this kernel at 48x101x101x8"
+                                               if conv_pipe else "not profiled at this slice shape"),
                           "face_updates_per_step": int((p_faces + r_faces) * conv_substeps)},
         "autotune": tune,
         "clocks": clk.summary(),

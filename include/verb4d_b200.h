@@ -285,6 +285,13 @@ int verb_autotune_local_solve(verb_ctx* ctx, double dt, double sub_dt, double* t
 #define VERB_CONV_FMA 1
 #define VERB_CONV_STREAM 2
 int verb_set_convection_arith(verb_ctx* ctx, int mode);
+/* The kernel that a convection pass of this context runs, by its arithmetic,
+ * the slice's shape and the number of slices: line jobs (one warp a group of
+ * lines), two stages over line segments, or one thread per line. */
+#define VERB_CONV_KERNEL_LINES 0
+#define VERB_CONV_KERNEL_STAGED 1
+#define VERB_CONV_KERNEL_STREAM 2
+int verb_convection_kernel(const verb_ctx* ctx, int* kernel);
 
 /* ---- Krylov form of the local (V,K) solve ----------------------------------
  * verb_local_krylov takes the same local step as verb_local but solves each

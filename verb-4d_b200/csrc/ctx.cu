@@ -503,6 +503,24 @@ size_t conv_scratch_size(const Dims& d)
     return b * sizeof(double);
 }
 
+// The kernel of a convection pass (VERB_CONV_KERNEL_*): the two-stage one where
+// both sweeps run, a slice's planes fit the shared memory and it is the faster
+// (cg_faster); other shapes take one thread per line (stream mode) or the
+// line-job kernels of convection.cu.
+int conv_kernel_for(const verb_ctx* c, int& kernel)
+{
+    const Dims& d = c->d;
+    const long long slices = (long long)d.V * d.K;
+    const bool staged = c->conv_arith == VERB_CONV_STREAM ? conv_staged_check(d.P, d.R, slices) == VERB_OK
+                        : c->conv_arith == VERB_CONV_EXACT
+                            ? conv_staged_check_exact(d.P, d.R, slices) == VERB_OK : false;
+    const bool stream = c->conv_arith == VERB_CONV_STREAM && conv_stream_check(d.P, d.R) == VERB_OK;
+    if (!stream)
+        if (int s = (c->conv_arith == VERB_CONV_EXACT ? conv_check : conv_check_fma)(d.P, d.R)) return s;
+    kernel = staged ? VERB_CONV_KERNEL_STAGED : stream ? VERB_CONV_KERNEL_STREAM : VERB_CONV_KERNEL_LINES;
+    return VERB_OK;
+}
+
 int conv_run(verb_ctx* c, double dt)
 {
     const Dims& d = c->d;
@@ -520,16 +538,9 @@ int conv_run(verb_ctx* c, double dt)
         int s = need_bc(c, b);
         if (s) return s;
     }
-    // the two-stage kernel where both sweeps run, a slice's planes fit the shared
-    // memory and it is the faster one (cg_faster); other shapes take one thread
-    // per line (stream mode) or the line-job kernels of convection.cu
     const long long slices = (long long)d.V * d.K;
-    const bool staged = c->conv_arith == VERB_CONV_STREAM ? conv_staged_check(d.P, d.R, slices) == VERB_OK
-                        : c->conv_arith == VERB_CONV_EXACT
-                            ? conv_staged_check_exact(d.P, d.R, slices) == VERB_OK : false;
-    const bool stream = c->conv_arith == VERB_CONV_STREAM && conv_stream_check(d.P, d.R) == VERB_OK;
-    if (!stream)
-        if (int s = (c->conv_arith == VERB_CONV_EXACT ? conv_check : conv_check_fma)(d.P, d.R)) return s;
+    int kernel = 0;
+    if (int s = conv_kernel_for(c, kernel)) return s;
     // no more CTAs than slices
     auto cap = [&](int ctas) { return (int)std::min<size_t>(ctas, (size_t)d.V * d.K); };
     if (!c->conv_nctas) {
@@ -564,11 +575,11 @@ int conv_run(verb_ctx* c, double dt)
     a.status = c->status;
     PhaseTimer t(c, PH_CONV);
     CK(cudaMemsetAsync(c->ticket, 0, sizeof(int), c->stream));
-    if (staged && c->conv_arith == VERB_CONV_EXACT)
+    if (kernel == VERB_CONV_KERNEL_STAGED && c->conv_arith == VERB_CONV_EXACT)
         launch_convection_staged_exact(a, conv_staged_ctas_exact(d.P, d.R, slices), c->stream);
-    else if (staged)
+    else if (kernel == VERB_CONV_KERNEL_STAGED)
         launch_convection_staged(a, conv_staged_ctas(d.P, d.R, slices), c->stream);
-    else if (stream)
+    else if (kernel == VERB_CONV_KERNEL_STREAM)
         launch_convection_stream(a, cap(conv_stream_ctas(d.P, d.R)), c->stream);
     else if (c->conv_arith == VERB_CONV_EXACT)
         launch_convection(a, c->conv_nctas, c->stream);
@@ -1030,6 +1041,12 @@ int verb_autotune_local_solve(verb_ctx* c, double dt, double sub_dt, double* tim
     }
     if (chosen) *chosen = best;
     return VERB_OK;
+}
+
+int verb_convection_kernel(const verb_ctx* c, int* kernel)
+{
+    if (!c || !kernel) return VERB_ERR_ARG;
+    return conv_kernel_for(c, *kernel);
 }
 
 int verb_set_convection_arith(verb_ctx* c, int mode)

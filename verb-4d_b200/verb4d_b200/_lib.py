@@ -22,6 +22,7 @@ STATUS_NAMES = {
 }
 VERB_GUESS_ZERO, VERB_GUESS_PREV, VERB_GUESS_CNN = 0, 1, 2
 CONV_ARITH = {"exact": 0, "fma": 1, "stream": 2}
+CONV_KERNELS = ("lines", "staged", "stream")
 GUESS_IDS = {"zero": VERB_GUESS_ZERO, "prev": VERB_GUESS_PREV, "cnn": VERB_GUESS_CNN}
 
 
@@ -95,6 +96,7 @@ SIGNATURES = {
     "verb_precond_loss_grad": (C.c_int, [_vp, _vp, _vp, C.c_int, C.c_int, C.c_int, C.c_int, _vp,
                                          C.POINTER(C.c_float), _vp]),
     "verb_set_convection_arith": (C.c_int, [_vp, C.c_int]),
+    "verb_convection_kernel": (C.c_int, [_vp, _ip]),
     "verb_set_step_graph": (C.c_int, [_vp, C.c_int]),
     "verb_local_solve_variants": (C.c_int, [C.POINTER(C.c_int)]),
     "verb_local_solve_variant": (C.c_int, [C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int),

@@ -133,6 +133,13 @@ class Context:
         else runs the "fma" kernel)."""
         L.check(self.lib.verb_set_convection_arith(self.h, L.CONV_ARITH[mode]), "conv_arith")
 
+    def convection_kernel(self) -> str:
+        """The kernel a convection pass runs: "lines" (line jobs), "staged" (two
+        stages over line segments) or "stream" (one thread per line)."""
+        k = C.c_int(0)
+        L.check(self.lib.verb_convection_kernel(self.h, C.byref(k)), "convection_kernel")
+        return L.CONV_KERNELS[k.value]
+
     def local_krylov(self, dt: float, sub_dt: float, guess: str = "prev", cnn=None,
                      smooth: int = 0, omega: float = 2.0 / 3.0, max_outer: int = 10,
                      inner_maxit: int = 100, inner_tol: float = 1e-3,
