@@ -1098,6 +1098,23 @@ size_t conv_smem_bytes(int P, int R)
 
 size_t conv_scratch_doubles(int P, int R) { return conv_scratch_per_cta(P, R); }
 
+// A round of jobs of T cells a lane takes what the table gives, 0.8 of it with
+// one warp on a scheduler; measured, exact form: 5.3-5.6 us for 12 x 13 to 16 x 16
+// (T = 1 in both sweeps), 7.3-7.7 for 12 x 20 to 12 x 32 (T = 2), 8.7-8.9 for 18 x 20 to
+// 20 x 24 (T = 3), 10.8-11.5 for 26 x 26 to 30 x 30 (T = 4); the sums hold to 7 % up to
+// 44 x 22 (15.5).
+double conv_lines_chain(int P, int R)
+{
+    const double us[6] = {2.75, 3.75, 4.4, 5.7, 6.4, 7.3};
+    const SweepCfg cfg[2] = {sweep_cfg(P, R - 1), sweep_cfg(R, P)};
+    double t = 0.0;
+    for (const SweepCfg& c : cfg) {
+        const double round = c.T <= 6 ? us[c.T - 1] : us[5] + 0.9 * (c.T - 6);
+        for (int left = c.njobs; left > 0; left -= C3_WARPS) t += left > 4 ? round : 0.8 * round;
+    }
+    return t;
+}
+
 int conv_check(int P, int R)
 {
     if ((P >= 3 && sweep_cfg(P, R - 1).lpl == 0) || (R >= 3 && sweep_cfg(R, P).lpl == 0))

@@ -61,6 +61,7 @@ __host__ __device__ inline int cg_rs(int R) { return (R + 2 * CG_GH) | 1; }
 // Launch shape of a [P][R] slice.
 struct StagedShape {
     int threads;      // per CTA
+    int own;          // most cells of a segment
     int segP, segR;   // segments of an MLT line, of an L line
 };
 
@@ -677,42 +678,66 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
 // pass of three runs at once) 2.7 (1.08) ms, against 2.8 (1.14) with four
 // slices, 2.2 (2.22) with 2 cells and one slice.
 //
-// Exact form, one slice on an SM at a time.  Alone (and per pass of three runs
-// at once), line-job kernel before the arrow: 12 x 13 x 31 x 31, 2 cells 1.11 (0.70)
-// -> 1.20 (0.54) ms; 24 x 25 x 31 x 31, 5 cells 4.00 (2.59) -> 3.60 (1.82), with 2
-// cells 3.42 (3.40), 8 cells 4.80 (2.48); 13 x 90 x 31 x 31, 8 cells 3.68 (2.55) ->
-// 3.57 (2.43), 5 cells 2.98 (2.91); 24 x 51 x 31 x 31, 8 cells 6.69 (4.34) -> 6.03
-// (4.16); 48 x 51 x 45 x 21, 5 cells (and up to 512 threads) 23.5 (14.9) -> 13.9
-// (13.6); 48 x 101 x 61 x 13 40.7 (21.7) -> 24.4 (20.4).  With two slices on an SM
-// the slices of the most sub-steps slow each other: 24 x 51 alone 7.5 ms.
-//
-// That is for up to CG_WAVE slices an SM, where a pass waits for those slices.
-// Beyond, the slices there are decide: small ones take one more on an SM for each
-// CG_WAVE (24 x 25 x 47 x 31 4.19 (3.66) -> 3.97 (2.71) ms with two, 5.34 with one;
-// 24 x 25 x 61 x 61 9.03 (9.00) -> 6.58 (6.53) with three, 13.7 with one; 12 x 13 x
-// 61 x 61 2.47 (2.45) -> 1.57 (1.56)).  Where registers leave no room for three, the
-// line-job kernel is as fast or faster then and runs: 24 x 51 x 61 x 61 15.4 ms
-// against 22.9 with one slice on an SM, 24 x 51 x 47 x 31 6.83 (6.23) against 7.44
-// (6.03) with two; from 1800 points on only past 1.5 CG_WAVE: 36 x 76 x 47 x 31 20.9
-// (19.1) -> 18.8 (18.6), but 36 x 76 x 61 x 31 23.6 (23.6) against 24.1 (24.0), and
-// 48 x 101 x 61 x 61 94.8 against 95.6.  Slices below 400 points that come two an SM
-// or fewer are left to it too: 12 x 13 x 11 x 11 0.92 (0.35) against 1.05 (0.39).
+// Exact form, one slice on an SM at a time.  Times below are of a pass alone (and
+// per pass of three runs at once).
+//  * Up to 2.5 slices an SM, segments of 2 cells: the shortest chain, and there are
+//    not slices enough to fill the chip otherwise.  323 slices: 24 x 25 3.32 (1.38) with
+//    5 cells -> 3.23 (1.36) ms, 23 x 32 3.92 (1.66) -> 3.35 (1.41), 24 x 42 5.04 (2.37) with
+//    8 cells -> 4.13 (1.75); 620 slices, 22 x 19: 3.04 (1.34) with 5 cells, 2.45 (1.72) with 2.
+//  * Beyond, segments as long as they may be without the chain growing much: below
+//    400 points 2 cells (12 x 13 x 31 x 31 1.18 (0.51) ms, 5 cells 1.81 (0.73)), below
+//    1000 5 cells (24 x 25 x 31 x 31 3.58 (1.81), 2 cells 3.37 (3.37), 8 cells 4.80 (2.48)),
+//    below 1800 8 cells (24 x 51 x 31 x 31 6.03 (3.98), 5 cells 4.52 (4.49)), larger
+//    ones 5 or what 512 threads take (48 x 101 x 31 x 31, 14 cells, 25.3 (25.1)).
+//    Two slices on an SM slow the ones of the most sub-steps: 12 x 13 x 31 x 20 1.04 ms
+//    alone with one, 1.16 with two.
+//  * Up to CG_WAVE slices an SM a pass alone waits for the slices of the most
+//    sub-steps, and the kernel with the shorter sub-step is taken (cg_faster): for
+//    short lines that is the line-job kernel.  961 slices, this kernel against that one: 12 x 13
+//    1.18 (0.51) against 1.07 (0.70) ms, 16 x 16 1.60 (0.72) against 1.39 (0.90), 22 x 19
+//    3.31 (1.57) against 3.07 (2.02), 23 x 32 4.16 (2.64) against 3.90 (2.59); but 12 x 20
+//    1.23 (0.56) against 1.36 (0.90), 24 x 25 3.58 (1.81) against 3.80 (2.57), 26 x 26 4.30
+//    (2.74) against 4.56 (3.10), 44 x 22 7.92 (7.91) against 11.0 (7.04); from 1000 points
+//    on always this one: 24 x 51 6.03 (3.98) against 6.38 (4.28), 36 x 40 9.02 (8.98) against
+//    12.4 (7.72), 48 x 101 25.3 (25.1) against 40.4 (26.6).
+//  * The line-job kernel keeps what it wins so to 13 slices an SM, where it has no
+//    waiting left to fill: 1891 slices, 16 x 16 1.71 (1.37) against 1.60 (1.59), 22 x 19
+//    3.56 (2.45) against 3.55 (3.57); 3721, 16 x 16 2.62 (2.62) against 3.12 (3.12).
+//  * Else beyond CG_WAVE the slices there are decide: small ones take one more on an
+//    SM for each CG_WAVE (24 x 25 x 47 x 31 4.19 (3.66) -> 3.97 (2.71) ms with two, 5.34
+//    with one; 24 x 25 x 61 x 61 8.95 (8.96) -> 6.52 (6.48) with three, 13.7 with one).
+//    Where registers leave no room for three, the line-job kernel is as fast or faster and
+//    runs: 24 x 51 x 61 x 61 15.4 ms against 22.9 with one slice on an SM, 24 x 51 x 47 x 31
+//    6.83 (6.23) against 7.44 (6.03) with two; from 1800 points on only past 1.5 CG_WAVE:
+//    36 x 76 x 45 x 30 20.6 (17.0) -> 17.1 (17.0), but 36 x 76 x 61 x 31 23.0 (23.0) against
+//    24.1 (24.0), and 48 x 101 x 61 x 61 93.2 against 94.2.
 constexpr int CG_MAXT = 512;
+
+int cg_sms()
+{
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
 #ifdef VERB_BUILD_CONV_EXACT
-int cg_own(int P, int R)
+int cg_own(int P, int R, long long slices)
 {
     const int n = P * R;
-    return n < 400 ? 2 : (n >= 1000 && n < 1800 ? 8 : 5);
+    if (n < 400 || 2 * slices <= 5 * (long long)cg_sms()) return 2;
+    return n >= 1000 && n < 1800 ? 8 : 5;
 }
 constexpr int CG_STEP = 3, CG_WAVE = 8;
 #else
-int cg_own(int P, int R) { return P * R < 1200 ? 5 : 11; }
+int cg_own(int P, int R, long long) { return P * R < 1200 ? 5 : 11; }
 constexpr int CG_STEP = 6;
 #endif
 
-bool cg_shape(int P, int R, StagedShape& s)
+bool cg_shape(int P, int R, long long slices, StagedShape& s)
 {
-    for (int own = cg_own(P, R); own <= CG_MAX_OWN; own += CG_STEP) {
+    for (int own = cg_own(P, R, slices); own <= CG_MAX_OWN; own += CG_STEP) {
+        s.own = own;
         s.segP = (P - 1 + own - 1) / own;
         s.segR = (R - 1 + own - 1) / own;
         const int need = std::max((R - 1) * s.segP, P * s.segR);
@@ -737,23 +762,32 @@ StagedKernel cg_kernel(int P, int R, const StagedShape& s)
     return fn;
 }
 
-int cg_sms()
-{
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
-}
-
 // CTAs that an SM can hold
-int cg_resident(int P, int R)
+int cg_resident(int P, int R, long long slices)
 {
     int per = 0;
     StagedShape s;
-    if (!cg_shape(P, R, s)) return 1;
+    if (!cg_shape(P, R, slices, s)) return 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, cg_kernel(P, R, s), s.threads, cg_smem(P, R));
     return std::max(per, 1);
 }
+
+#ifdef VERB_BUILD_CONV_EXACT
+// us of a sub-step of one slice with segments of 2 or 5 cells: by the warps that a
+// sweep puts on a scheduler.  Measured for 2 cells: 6.0 us (12 x 13: one), 6.7 (17 x 17:
+// one and two), 7.4 (20 x 20), 9.1 (24 x 25: three), 11.4 (30 x 30: four); for 5: 9.1
+// (20 x 24), 10.3 (26 x 26: one and two), 11.4 (30 x 30: two), 13.3 (13 x 90: three).
+double cg_chain(int P, int R, const StagedShape& s)
+{
+    const double two[4] = {3.03, 3.7, 4.6, 5.7}, five[4] = {4.55, 5.7, 6.8, 8.0};
+    double t = 0.0;
+    for (int threads : {(R - 1) * s.segP, P * s.segR}) {
+        const int w = ((threads + 31) / 32 + 3) / 4;  // 1 .. 4: up to CG_MAXT threads
+        t += (s.own == 2 ? two : five)[w - 1];
+    }
+    return t;
+}
+#endif
 
 // Whether this kernel is the faster one for so many slices (the contracted form
 // always is: 1.2 to 4 times from 12 x 13 to 48 x 101, 961 and 3721 slices)
@@ -761,9 +795,11 @@ bool cg_faster(int P, int R, long long slices)
 {
 #ifdef VERB_BUILD_CONV_EXACT
     const long long n = (long long)P * R, sms = cg_sms();
-    if (n < 400 && slices <= 2 * sms) return false;
-    if (2 * slices <= (n < 1800 ? 2 : 3) * CG_WAVE * sms) return true;
-    return n < 1000 && cg_resident(P, R) >= 3;
+    if (n >= 1000) return 2 * slices <= (n < 1800 ? 2 : 3) * CG_WAVE * sms;
+    StagedShape s;
+    cg_shape(P, R, slices, s);
+    if (slices <= 13 * sms && conv_lines_chain(P, R) < cg_chain(P, R, s)) return false;
+    return slices <= CG_WAVE * sms || cg_resident(P, R, slices) >= 3;
 #else
     return true;
 #endif
@@ -778,7 +814,7 @@ int VERB_STAGED(conv_staged_check)(int P, int R, long long slices)
 {
     if (P < 11 || R < 11) return VERB_ERR_SIZE;
     StagedShape s;
-    if (!cg_shape(P, R, s) ||
+    if (!cg_shape(P, R, slices, s) ||
         cg_smem(P, R) > allow_max_dynamic_smem((const void*)cg_kernel(P, R, s)))
         return VERB_ERR_SIZE;
     return cg_faster(P, R, slices) ? VERB_OK : VERB_ERR_SIZE;
@@ -789,7 +825,7 @@ size_t VERB_STAGED(conv_staged_scratch_doubles)(int P, int R) { return (cg_scrat
 int VERB_STAGED(conv_staged_ctas)(int P, int R, long long slices)
 {
     const int sms = cg_sms();
-    long long per = cg_resident(P, R);
+    long long per = cg_resident(P, R, slices);
 #ifdef VERB_BUILD_CONV_EXACT
     per = std::min(per, (slices + CG_WAVE * sms - 1) / (CG_WAVE * sms));
 #endif
@@ -799,7 +835,7 @@ int VERB_STAGED(conv_staged_ctas)(int P, int R, long long slices)
 void VERB_STAGED(launch_convection_staged)(const ConvArgs& a, int nctas, cudaStream_t st)
 {
     StagedShape s;
-    cg_shape(a.d.P, a.d.R, s);
+    cg_shape(a.d.P, a.d.R, (long long)a.d.V * a.d.K, s);
     const StagedKernel fn = cg_kernel(a.d.P, a.d.R, s);
     fn<<<nctas, s.threads, cg_smem(a.d.P, a.d.R), st>>>(a, s.segP, s.segR);
 }

@@ -111,6 +111,9 @@ struct ConvArgs {
 };
 int conv_ctas(int P, int R);
 int conv_check(int P, int R);  // VERB_ERR_SIZE for slices the kernel cannot hold
+// us of a sub-step of one slice in the line-job kernel: the rounds of jobs of both
+// sweeps (P, R >= 3)
+double conv_lines_chain(int P, int R);
 size_t conv_smem_bytes(int P, int R);
 size_t conv_scratch_doubles(int P, int R);
 void launch_convection(const ConvArgs& a, int nctas, cudaStream_t s);
