@@ -1098,7 +1098,7 @@ size_t conv_smem_bytes(int P, int R)
 
 size_t conv_scratch_doubles(int P, int R) { return conv_scratch_per_cta(P, R); }
 
-// A round of jobs of T cells a lane takes what the table gives, 0.8 of it with
+// A round of jobs of T cells a lane takes what the table gives, 0.85 of it with
 // one warp on a scheduler; measured, exact form: 5.3-5.6 us for 12 x 13 to 16 x 16
 // (T = 1 in both sweeps), 7.3-7.7 for 12 x 20 to 12 x 32 (T = 2), 8.7-8.9 for 18 x 20 to
 // 20 x 24 (T = 3), 10.8-11.5 for 26 x 26 to 30 x 30 (T = 4); the sums hold to 7 % up to
@@ -1110,7 +1110,7 @@ double conv_lines_chain(int P, int R)
     double t = 0.0;
     for (const SweepCfg& c : cfg) {
         const double round = c.T <= 6 ? us[c.T - 1] : us[5] + 0.9 * (c.T - 6);
-        for (int left = c.njobs; left > 0; left -= C3_WARPS) t += left > 4 ? round : 0.8 * round;
+        for (int left = c.njobs; left > 0; left -= C3_WARPS) t += left > 4 ? round : 0.85 * round;
     }
     return t;
 }
