@@ -10,10 +10,10 @@
 // coefficients change (src/VERB4D_Solver.cpp:1091-1096).
 //
 // Kernels:
-//  * local_factor_kernel: one CTA per system (V < 7 and grids of more than
-//    65535 systems).  Rows of A are assembled on the
-//    device with the reference's operation order (bit-identical matrix) and
-//    factored by the unblocked banded LU of LAPACK's xGBTF2 (partial pivoting,
+//  * local_factor_kernel: one CTA per system, where local_factor_blk_kernel does
+//    not run (V <= 7, with FP32 factors V <= 15, and grids of more than 65535
+//    systems: factor_by_panels).  Rows of A are assembled on the device with the
+//    reference's operation order (bit-identical matrix) and factored by the unblocked banded LU of LAPACK's xGBTF2 (partial pivoting,
 //    multipliers scaled by the reciprocal pivot, rank-1 updates as fused
 //    multiply-adds).
 //    The active (kl+1) x (kv+1) window lives in shared memory as a circular
@@ -1999,13 +1999,17 @@ void launch_factor_blk(const LocalArgs& a, cudaStream_t s)
     local_factor_blk_kernel<T, PW, NW><<<a.d.P * a.d.R, NW * 32, smem, s>>>(a, f);
 }
 
+// Whether the panel kernel takes the systems: a parked row needs 9 doubles of an
+// L column (V >= 8, in FP32 V >= 16), and systems index grid.y of the parking launch.
+bool factor_by_panels(const LocalArgs& a)
+{
+    return (a.factors32 ? a.klp32 >= 18 : a.klp >= 9) && a.d.P * a.d.R <= 65535;
+}
+
 template <typename T>
 bool launch_factor_blk_t(const LocalArgs& a, cudaStream_t s)
 {
-    // a parked row needs 9 doubles of an L column; systems index grid.y of
-    // the parking launch
-    if (a.factors32 ? a.klp32 < 18 : a.klp < 9) return false;
-    if (a.d.P * a.d.R > 65535) return false;
+    if (!factor_by_panels(a)) return false;
     // PW: the kl + NB rows of a panel, one a thread; the warps beside them share
     // the update.  Measured while the kernel was built, an upload-factorise-solve
     // pass: 24 x 51 x 101 x 21 with 4 + 8 warps 18.9 ms (4 + 12: 19.3, 4 + 4: 22.9;
@@ -2026,8 +2030,7 @@ int launch_local_factor(const LocalArgs& a, cudaStream_t s)
     // The blocked kernel writes every entry of Uf (above row 0 and the padding
     // included) of the systems it factors; where some are skipped, and for the
     // window kernel, Uf is cleared first.
-    const bool blk = a.factors32 ? a.klp32 >= 18 : a.klp >= 9;
-    if (!(blk && a.d.P * a.d.R <= 65535) || !a.include_boundary || a.k0 || a.sel)
+    if (!factor_by_panels(a) || !a.include_boundary || a.k0 || a.sel)
         cudaMemsetAsync(a.factors32 ? (void*)a.Uf32 : (void*)a.Uf, 0,
                         a.unknowns * (a.factors32 ? a.kvp32 * sizeof(float) : a.kvp * sizeof(double)), s);
     if (a.factors32 ? launch_factor_blk_t<float>(a, s) : launch_factor_blk_t<double>(a, s)) return 2;
