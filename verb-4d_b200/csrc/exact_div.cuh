@@ -6,11 +6,11 @@
 namespace verb {
 namespace {
 
-// RN(1 / x) for 2^-1000 < |x| < 2^1000: Newton steps from the hardware's
-// approximation, the last one correcting by the exact residual, which rounds
-// correctly except where the significand of x is all ones (Markstein, IBM J.
-// Res. Dev. 34, 1990); there 1/x lies just above the midpoint of a power of
-// two and its successor and rounds to the successor.
+// RN(1 / x) for 2^-1021 <= |x| < 2^1022, where x, 1/x and the steps stay normal:
+// Newton steps from the hardware's approximation, the last one correcting by the
+// exact residual, which rounds correctly except where the significand of x is all
+// ones (Markstein, IBM J. Res. Dev. 34, 1990); there 1/x lies just above the
+// midpoint of a power of two and its successor and rounds to the successor.
 __device__ __forceinline__ double recip(double x)
 {
     double y;
