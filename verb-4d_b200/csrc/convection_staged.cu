@@ -676,7 +676,13 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
 // face by face 29.8).  Below 1200 points a pass waits for the slices of the most
 // sub-steps: 5 cells and two slices on an SM, 24 x 25 x 31 x 31 alone (and per
 // pass of three runs at once) 2.7 (1.08) ms, against 2.8 (1.14) with four
-// slices, 2.2 (2.22) with 2 cells and one slice.
+// slices, 2.2 (2.22) with 2 cells and one slice.  Around the line, 5 cells against
+// 11: 961 slices, 24 x 32 3.07 (1.77) against 4.61 (1.81), 24 x 48 3.80 (2.14) against 4.50
+// (2.54), and beyond it 24 x 51 3.84 (2.11) against 5.59 (2.36), 36 x 50 5.16 (5.11)
+// against 9.20 (5.25); 3721 slices, 24 x 40 7.14 (7.09) against 6.42 (6.34), 24 x 48 7.52
+// (7.48) against 9.15 (9.10), and beyond it 30 x 42 14.6 (14.6) against 8.40 (7.79), 36 x 50
+// 19.3 (19.2) against 18.3 (18.3): with slices as few, one run would have 5 cells
+// above the line as well.
 //
 // Exact form, one slice on an SM at a time.  Times below are of a pass alone (and
 // per pass of three runs at once).

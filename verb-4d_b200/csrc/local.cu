@@ -2011,10 +2011,14 @@ bool launch_factor_blk_t(const LocalArgs& a, cudaStream_t s)
 {
     if (!factor_by_panels(a)) return false;
     // PW: the kl + NB rows of a panel, one a thread; the warps beside them share
-    // the update.  Measured while the kernel was built, an upload-factorise-solve
-    // pass: 24 x 51 x 101 x 21 with 4 + 8 warps 18.9 ms (4 + 12: 19.3, 4 + 4: 22.9;
-    // panels of 16 columns 19.5-21.5), 24 x 25 x 31 x 31 with 2 + 2 warps 3.6 ms
-    // alone (2 + 4: 4.0; 16 columns 4.2).
+    // the update.  The factorisation alone, ms by the warps in all:
+    //   V = 16, 24 x 25 x 31:  2 0.451, 3 0.434, 4 0.447, 5 0.637 (FP32 0.447, 0.427, 0.440, 0.634)
+    //   V = 31, 24 x 25 x 31:  3 1.116, 4 1.017, 6 1.088; V = 50: 3 2.62, 4 1.95, 6 1.76
+    //   V = 60, 24 x 25 x 21:  6 2.49, 9 2.93, 12 2.87; V = 80, 24 x 25 x 15: 6 5.43, 9 4.56, 12 4.36
+    //   V = 101, 24 x 51 x 21, the pass with upload and solve: 8 22.9, 12 18.9, 16 19.3 (16.1 by
+    //   now with 12)
+    // and panels of 16 columns instead of 8: V = 101 19.5-21.5 ms, V = 31 the pass of one run
+    // 4.2 against 3.6.
     const int kl = a.d.V + 1;
     if (kl + NB <= 32) launch_factor_blk<T, 1, 3>(a, s);
     else if (kl + NB <= 64) launch_factor_blk<T, 2, 4>(a, s);
