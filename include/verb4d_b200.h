@@ -270,15 +270,17 @@ int verb_autotune_local_solve(verb_ctx* ctx, double dt, double sub_dt, double* t
  * reference's operations one by one without contraction, so results are
  * bit-identical to it (exp() of loss rates aside).  VERB_CONV_FMA runs the
  * line-job kernel compiled with multiply-add contraction, within a few units
- * in the last place of the exact form per step.  VERB_CONV_STREAM is
- * contracted too, with the G product and the loss/source epilogue applied as
- * the sweeps store, and the fastest; it needs both sweeps (P and R >= 11) and
- * otherwise runs the VERB_CONV_FMA kernel; within a few units in the last
- * place of the reference per step.  With both sweeps, VERB_CONV_EXACT and
- * VERB_CONV_STREAM run the two-stage kernel over line segments where its three
- * planes fit in shared memory (VERB_CONV_EXACT: and unless slices are so many
- * that the line-job kernel is faster), else the line-job kernel and the kernel
- * with one thread per line.  Convection_2D
+ * in the last place of the exact form per step; it is the faster of the two
+ * where exact runs the line-job kernel too.  VERB_CONV_STREAM is contracted
+ * as well, with the G product and the loss/source epilogue applied as the
+ * sweeps store, and the fastest for all but a few small numbers of slices; it
+ * needs both sweeps (P and R >= 11) and otherwise runs the VERB_CONV_FMA
+ * kernel; within a few units in the last place of the reference per step.
+ * With both sweeps, VERB_CONV_EXACT and VERB_CONV_STREAM run the two-stage
+ * kernel over line segments where its three planes fit in shared memory
+ * (VERB_CONV_EXACT: and unless lines are so short or slices so many that the
+ * line-job kernel is faster), else the line-job kernel and the kernel with one
+ * thread per line.  Convection_2D
  * (src/Convection_2D.cpp:36-169) has one arithmetic; the switch has no
  * counterpart in the reference. */
 #define VERB_CONV_EXACT 0

@@ -128,9 +128,11 @@ class Context:
 
     def set_convection_arith(self, mode: str = "exact"):
         """"exact": bit-identical to the reference; "fma": multiply-add
-        contraction of the line-job kernel, a few ulp per step from "exact";
-        "stream": the fastest, contracted like "fma" (needs P and R >= 11,
-        else runs the "fma" kernel)."""
+        contraction of the line-job kernel, a few ulp per step from "exact"
+        and faster than it where that runs line jobs too
+        (:meth:`convection_kernel`); "stream": contracted like "fma" and the
+        fastest for all but a few small numbers of slices (needs P and
+        R >= 11, else runs the "fma" kernel)."""
         L.check(self.lib.verb_set_convection_arith(self.h, L.CONV_ARITH[mode]), "conv_arith")
 
     def convection_kernel(self) -> str:
