@@ -427,13 +427,14 @@ __device__ __forceinline__ void frw_wait_all() { asm volatile("cp.async.wait_all
 // in that order: bit-equal to the fma chain), and a row's multipliers move
 // with the row when a later pivot of the panel interchanges it.  Factors and
 // pivots are therefore bit-identical to it.  xGBTF2 skips the update where
-// u_kc = 0; adding a zero product leaves a finite element as it is, so the
-// skip is only taken where a panel holds a zero or tiny pivot or a value that
-// is not finite (the slow branches below).
+// u_kc = 0 and updates the rows within kl of the pivot only, those of zero
+// multipliers included; adding a zero product leaves a finite element as it is,
+// so both matter only where a panel holds a zero or tiny pivot or a value above
+// 2^1000 or not finite (the slow branches below).
 //
 // 24 x 51 x 101 x 21 (1224 systems, factors 12.9 GB), the pass with the solve:
-// 60.5 ms with the unblocked register-window kernel this replaces, 16.1 ms here;
-// 24 x 25 x 31 x 31, the mixed form's pass: 4.76 -> 1.53 ms, 0.94 of it here.  The
+// 60.5 ms with the unblocked register-window kernel this replaces, 15.5 ms here;
+// 24 x 25 x 31 x 31, the mixed form's pass: 4.76 -> 1.48 ms, 0.9 of it here.  The
 // bound is the panel: about 1000 cycles a column of pivot search and exchange
 // through shared memory, against 160-320 for the multiply-adds of the update,
 // which run beside it; writing the factors at the copy bandwidth takes 2 ms.
@@ -467,8 +468,14 @@ __device__ __forceinline__ void sts2_if(bool c, double* p, double x, double y)
         : "memory");
 }
 
+// Blocks an SM is to hold (registers up to 96, 96 and 112; the window's shared memory
+// allows them for the bands that PW serves): left to itself the compiler takes 126
+// registers for PW = 1 and 2, and 24 x 25 x 31 x 31 comes in two waves, 1.88 against 1.53
+// ms for the pass.
+constexpr int fb_min_blocks(int PW) { return PW == 1 ? 6 : PW == 2 ? 5 : PW == 3 ? 2 : 1; }
+
 template <typename T, int PW, int NW>
-__global__ void __launch_bounds__(NW * 32) local_factor_blk_kernel(LocalArgs a, FBlk f)
+__global__ void __launch_bounds__(NW * 32, fb_min_blocks(PW)) local_factor_blk_kernel(LocalArgs a, FBlk f)
 {
     extern __shared__ __align__(16) double sm[];
     const int sys = blockIdx.x;
@@ -486,6 +493,9 @@ __global__ void __launch_bounds__(NW * 32) local_factor_blk_kernel(LocalArgs a, 
     // a panel's interchanges as one permutation of the rows (window offsets):
     // row k <- row s_src[k], and s_no rows below the panel <- rows of it
     __shared__ int s_src[2][NB], s_od[2][NB], s_os[2][NB], s_no[2];
+    // for the slow branches: row k's position before the panel, and the last such
+    // position that the panel's pivot k updates (-1: it is zero and updates nothing)
+    __shared__ int s_init[2][NB], s_lim[2][NB];
     __shared__ int s_ju[2];                        // last column a panel's pivot rows reach
     __shared__ int s_bad[2];                       // a non-finite multiplier in the panel
     __shared__ int s_badu;                         // a non-finite U entry
@@ -558,6 +568,7 @@ __global__ void __launch_bounds__(NW * 32) local_factor_blk_kernel(LocalArgs a, 
             s_no[par] = 0;
             s_huge = 0;
         }
+        if (tid < NB) s_lim[par][tid] = min(tid + kl, n - 1 - j0);
         named_sync(2, PT);
         if (top >= 0x7e700000u) s_huge = 1;
         int jj = 0;
@@ -671,7 +682,10 @@ __global__ void __launch_bounds__(NW * 32) local_factor_blk_kernel(LocalArgs a, 
                 }
                 if (tid == 0) {
                     ip[j] = j0 + p;
-                    if (!nz) set_error(a.status, VERB_ERR_PIVOT);
+                    if (!nz) {
+                        s_lim[par][jj] = -1;
+                        set_error(a.status, VERB_ERR_PIVOT);
+                    }
                 }
                 named_sync(2, PT);
                 const double rcp = 1.0 / piv;
@@ -697,7 +711,10 @@ __global__ void __launch_bounds__(NW * 32) local_factor_blk_kernel(LocalArgs a, 
             tri[(par * NB + m) * NB + i] = i && m + i < NB ? -W[off(m + i) + slot(m)] : 0.0;
         }
         // the interchanges as one permutation
-        if (pos < NB) s_src[par][pos] = off(t);
+        if (pos < NB) {
+            s_src[par][pos] = off(t);
+            s_init[par][pos] = t;
+        }
         if (pos >= NB && pos != t) {
             const int i = atomicAdd(&s_no[par], 1);
             s_od[par][i] = off(pos);
@@ -747,8 +764,12 @@ __global__ void __launch_bounds__(NW * 32) local_factor_blk_kernel(LocalArgs a, 
             for (; c < c_hi; c += step) {
                 double* col = W + cslot(c);
                 double x[NB];
+                unsigned top = 0;
 #pragma unroll
-                for (int k = 0; k < NB; k++) x[k] = col[s_src[par][k]];
+                for (int k = 0; k < NB; k++) {
+                    x[k] = col[s_src[par][k]];
+                    top = max(top, (unsigned)__double2hiint(x[k]) & 0x7fffffffu);
+                }
 #pragma unroll 1
                 for (int i = 0; i < no; i += 4) {
                     double y[4];
@@ -758,10 +779,27 @@ __global__ void __launch_bounds__(NW * 32) local_factor_blk_kernel(LocalArgs a, 
                     for (int e = 0; e < 4; e++)
                         if (i + e < no) col[s_od[par][i + e]] = y[e];
                 }
-                unsigned top = 0;
                 int r = rj;
+                if (__builtin_expect(slow || top >= 0x7e700000u, 0)) {
+                    // operation by operation as xGBTF2 does it: a pivot of the
+                    // panel updates the rows it reaches, unless its u is zero
+#pragma unroll
+                    for (int k = 0; k < NB; k++) col[rslot(k)] = x[k];
+#pragma unroll 1
+                    for (int m = 0; m < NB; m++) {
+                        const double u = col[rslot(m)];
+                        if (((unsigned)__double2hiint(u) & 0x7fffffffu) >= 0x7ff00000u) s_badu = 1;
+                        if (u == 0.0) continue;
+#pragma unroll 1
+                        for (int k = m + 1; k < NB; k++)
+                            if (s_init[par][k] <= s_lim[par][m])
+                                col[rslot(k)] = fma(tr[m * NB + k - m], u, col[rslot(k)]);
+                    }
+                    continue;
+                }
                 // row m is always x[0]: the loop stays rolled; the next
-                // multipliers are loaded while these are used
+                // multipliers are loaded while these are used.  Values up to 2^1000
+                // stay finite (|l| <= 1)
                 double2 l[NB / 2];
 #pragma unroll
                 for (int k = 0; k < NB / 2; k++) l[k] = *(const double2*)(tr + 2 * k);
@@ -770,17 +808,15 @@ __global__ void __launch_bounds__(NW * 32) local_factor_blk_kernel(LocalArgs a, 
                     const double u = x[0];
                     col[r * pitch] = u;
                     r = r + 1 == RW ? 0 : r + 1;
-                    top = max(top, (unsigned)__double2hiint(u) & 0x7fffffffu);
                     const double* tn = tr + min(m + 1, NB - 1) * NB;
 #pragma unroll
                     for (int k = 0; k < NB / 2; k++) {
                         const double2 lk = l[k];
                         l[k] = *(const double2*)(tn + 2 * k);
-                        if (k) x[2 * k - 1] = slow && u == 0.0 ? x[2 * k] : fma(lk.x, u, x[2 * k]);
-                        x[2 * k] = slow && u == 0.0 ? x[2 * k + 1] : fma(lk.y, u, x[2 * k + 1]);
+                        if (k) x[2 * k - 1] = fma(lk.x, u, x[2 * k]);
+                        x[2 * k] = fma(lk.y, u, x[2 * k + 1]);
                     }
                 }
-                if (top >= 0x7ff00000u) s_badu = 1;
             }
         };
         // The update of columns c_lo .. c_hi-1 (relative to j0): warp w of nw
@@ -834,17 +870,26 @@ __global__ void __launch_bounds__(NW * 32) local_factor_blk_kernel(LocalArgs a, 
                 }
             }
         };
-        // the same update element by element with xGBTF2's skip (rows a pivot
-        // does not reach hold a zero multiplier)
+        // the same update element by element as xGBTF2 does it: a pivot updates the
+        // rows it reaches, those of zero multipliers included, unless its u is zero
         auto update_slow = [&](int c_lo, int c_hi, int t, int nt) {
+#pragma unroll 1
             for (int e = t; e < (c_hi - c_lo) * kl; e += nt) {
-                const int c = c_lo + e / kl, r = NB + e % kl;
-                double v = W[rslot(r) + cslot(c)];
+                const int c = c_lo + e / kl, ro = rslot(NB + e % kl);
+                int init = NB + e % kl;  // the row's position before the panel
+#pragma unroll 1
+                for (int i = 0; i < s_no[par]; i++)
+                    if (s_od[par][i] == ro) {
+                        const int q = s_os[par][i] / pitch - rj;
+                        init = q < 0 ? q + RW : q;
+                    }
+                double v = W[ro + cslot(c)];
+#pragma unroll 1
                 for (int k = 0; k < NB; k++) {
-                    const double u = W[rslot(k) + cslot(c)], l = W[rslot(r) + cslot(k)];
-                    if (u != 0.0 && l != 0.0) v = fma(l, -u, v);
+                    const double u = W[rslot(k) + cslot(c)], l = W[ro + cslot(k)];
+                    if (u != 0.0 && init <= s_lim[par][k]) v = fma(l, -u, v);
                 }
-                W[rslot(r) + cslot(c)] = v;
+                W[ro + cslot(c)] = v;
             }
         };
 
@@ -2015,7 +2060,7 @@ bool launch_factor_blk_t(const LocalArgs& a, cudaStream_t s)
     //   V = 16, 24 x 25 x 31:  2 0.451, 3 0.434, 4 0.447, 5 0.637 (FP32 0.447, 0.427, 0.440, 0.634)
     //   V = 31, 24 x 25 x 31:  3 1.116, 4 1.017, 6 1.088; V = 50: 3 2.62, 4 1.95, 6 1.76
     //   V = 60, 24 x 25 x 21:  6 2.49, 9 2.93, 12 2.87; V = 80, 24 x 25 x 15: 6 5.43, 9 4.56, 12 4.36
-    //   V = 101, 24 x 51 x 21, the pass with upload and solve: 8 22.9, 12 18.9, 16 19.3 (16.1 by
+    //   V = 101, 24 x 51 x 21, the pass with upload and solve: 8 22.9, 12 18.9, 16 19.3 (15.5 by
     //   now with 12)
     // and panels of 16 columns instead of 8: V = 101 19.5-21.5 ms, V = 31 the pass of one run
     // 4.2 against 3.6.
