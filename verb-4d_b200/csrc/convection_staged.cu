@@ -130,6 +130,21 @@ __device__ __forceinline__ void line_ghosts(double* E, int st, int n, int lt, in
 // polynomials and the limiters of a group are independent of each other, and
 // the window is loaded once per group instead of shifted through registers.
 
+// Unlimited value of one face from its stencil e[k * st] = E[x-5+k], the
+// reference's sums as they stand
+__device__ __forceinline__ double face_alone(const double* e, int st, double c)
+{
+    const bool pos = c >= 0;
+    double a[5], b[5];  // upwind from the centre on, downwind
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        a[k] = e[(pos ? 4 - k : 5 + k) * st];
+        b[k] = e[(pos ? 5 + k : 4 - k) * st];
+    }
+    return quickest_face_k(a[1], a[2], a[3], a[4], a[0], b[0], b[1], b[2], b[3], b[4], c,
+                           face_coef_exact(c));
+}
+
 #ifdef VERB_BUILD_CONV_EXACT
 // Unlimited values of U faces from the window d[k] = E[x-5+k], the roles of the
 // stencil's points chosen by the direction (QUICKEST6.cpp:169-186)
@@ -156,7 +171,9 @@ __device__ __forceinline__ void faces(double (&d)[U + 9], const double (&c)[U], 
 // faces, D^m_k = D^(m-1)_k - D^(m-1)_(k+1), shared by neighbouring faces: with
 // (a, b) the two m-th differences at face u, m even, the reference's even term
 // is (a + b) / 2 and its odd term a - b.  The ninth-order pair E8 + sign d9 is
-// 2a or 2b.
+// 2a or 2b: it leaves out the stencil's last point, and (a + b) of two infinities is
+// not a number where the reference's sum is infinite, so slices that hold such
+// values are left to a second launch (ODD), whose faces are face_alone's.
 template <int U>
 __device__ __forceinline__ void faces(double (&d)[U + 9], const double (&c)[U], double (&f)[U])
 {
@@ -205,10 +222,15 @@ __device__ __forceinline__ void faces(double (&d)[U + 9], const double (&c)[U], 
         f[u] += (p[u] * (1.0 / 362880.0)) * (c[u] >= 0 ? d[u] : d[u + 1]);
 }
 
+// NaN, infinite or above 2^300
+__device__ __forceinline__ bool is_odd(double v)
+{
+    return ((unsigned)__double2hiint(v) & 0x7fffffffu) >= 0x52b00000u;
+}
 #endif
 
 // returns unlimited face a, whose slot is the neighbour's
-template <int U>
+template <int U, bool ODD>
 __device__ __forceinline__ double stage1(const Seg& L)
 {
     double Q = 0.0, f0 = 0.0;
@@ -218,14 +240,23 @@ __device__ __forceinline__ double stage1(const Seg& L)
 #pragma unroll 1
     for (int i = 0; i <= L.own; i += U) {
         const int x = L.a + i;
-        double d[U + 9], c[U], f[U];
+        double d[U + 9], c[U], f[U] = {};
 #pragma unroll
         for (int u = 0; u < U; u++) c[u] = cp[u * L.nl];
         cp += U * L.nl;
         const double* ep = L.E + (x - 5) * L.st;
 #pragma unroll
         for (int k = 0; k < U + 9; k++) d[k] = ep[k * L.st];
-        faces<U>(d, c, f);
+        if constexpr (ODD) {
+#pragma unroll 1
+            for (int u = 0; u < U; u++) {
+                const double v = face_alone(ep + u * L.st, L.st, cp[(u - U) * L.nl]);
+#pragma unroll
+                for (int k = 0; k < U; k++) f[k] = k == u ? v : f[k];
+            }
+        } else {
+            faces<U>(d, c, f);
+        }
         double* up = L.U + (x - 1) * L.st;
         double* fp = L.O + (x - 1) * L.st;
         if (i == 0) f0 = f[0];
@@ -444,7 +475,7 @@ __device__ __forceinline__ double cg_block_max(double v, double* red)
     return m;
 }
 
-template <int U1, int MAXT, int MINB>
+template <int U1, int MAXT, int MINB, bool ODD = false>
 __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs a, int segP, int segR)
 {
     extern __shared__ __align__(16) double sm[];
@@ -483,7 +514,12 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
 
     for (;;) {
         if (tid == 0) {
-            s_ticket = atomicAdd(a.ticket, 1);
+            if constexpr (ODD) {
+                const int q = atomicAdd(a.ticket + 2, 1);
+                s_ticket = q < a.ticket[1] ? a.odd[q] : nslices;
+            } else {
+                s_ticket = atomicAdd(a.ticket, 1);
+            }
             s_ns[0] = s_ns[1] = 1;
         }
         __syncthreads();
@@ -529,6 +565,7 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
         }
         const double dtc = a.dt / num_steps;
         if (tid == 0) a.substeps[off] = (int)num_steps;
+        bool odd = false;  // a value that is left to the second launch
         for (int i = tid; i < PR; i += nt) {
             const int iP = i / R, iR = i - iP * R;
             const size_t gi = g(iP, iR);
@@ -539,7 +576,9 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
             e3R[(size_t)iR * P + iP] = G;
             e4R[(size_t)iR * P + iP] = __drcp_rn(G);
 #else
-            e1R[(size_t)iR * P + iP] = exp(a.loss[gi] * dtc) / G;
+            const double eg = exp(a.loss[gi] * dtc) / G;
+            e1R[(size_t)iR * P + iP] = eg;
+            if (is_odd(S[iP * Rs + iR]) || is_odd(G) || is_odd(eg) || is_odd(a.S[gi])) odd = true;
 #endif
             e2R[(size_t)iR * P + iP] = iR && iR < R - 1 ? a.S[gi] * dtc : -0.0;
         }
@@ -584,6 +623,9 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
                 const size_t bo = ((size_t)iR * V + iV) * K + iK;
                 lnP[iR] = a.Pl[bo];
                 lnP[(R - 1) + iR] = a.Pu[bo];
+#ifndef VERB_BUILD_CONV_EXACT
+                if (a.Pl_t != VERB_BC_PERIODIC && (is_odd(a.Pl[bo]) || is_odd(a.Pu[bo]))) odd = true;
+#endif
             }
         }
         for (int iP = warp; iP < P; iP += nw) {
@@ -592,11 +634,22 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
                 const size_t bo = ((size_t)iP * V + iV) * K + iK;
                 lnR[iP] = a.Rl[bo] * a.G[g(iP, 0)];
                 lnR[P + iP] = a.Ru[bo] * a.G[g(iP, R - 1)];
+#ifndef VERB_BUILD_CONV_EXACT
+                if (a.Rl_t != VERB_BC_PERIODIC && (is_odd(lnR[iP]) || is_odd(lnR[P + iP]))) odd = true;
+#endif
             }
         }
+        double steps = num_steps;
+#ifdef VERB_BUILD_CONV_EXACT
         __syncthreads();
+#else
+        if (__syncthreads_or(odd) && !ODD) {  // (a jump out of here costs registers)
+            if (tid == 0) a.odd[atomicAdd(a.ticket + 1, 1)] = t;
+            steps = 0;
+        }
+#endif
 
-        for (int it = 0; it < num_steps; it++) {
+        for (int it = 0; it < steps; it++) {
             // the MLT sweep (ph 0: P-lines iR, stored times G) and the L sweep
             // (ph 1: R-lines iP, stored as v exp(Loss dt)/G + S dt) go through
             // one copy of the stages
@@ -639,7 +692,7 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
                     const bool run = k < ns, last = k == ns - 1;
                     double f0 = 0.0;
                     __syncthreads();
-                    if (run) f0 = stage1<U1>(L);
+                    if (run) f0 = stage1<U1, ODD>(L);
                     __syncthreads();
                     if (run) {
                         stage2(L, f0, last);
@@ -754,15 +807,16 @@ bool cg_shape(int P, int R, long long slices, StagedShape& s)
 }
 
 typedef void (*StagedKernel)(ConvArgs, int, int);
-StagedKernel cg_kernel(int P, int R, const StagedShape& s)
+StagedKernel cg_kernel(int P, int R, const StagedShape& s, bool odd = false)
 {
 #ifdef VERB_BUILD_CONV_EXACT
     StagedKernel fn = convection_staged_kernel<3, CG_MAXT, 1>;
     if (s.threads <= 320) fn = convection_staged_kernel<3, 320, 1>;
     if (s.threads <= 160) fn = convection_staged_kernel<3, 160, 2>;
 #else
-    StagedKernel fn = convection_staged_kernel<6, CG_MAXT, 1>;
-    if (P * R < 1200 && s.threads <= 160) fn = convection_staged_kernel<3, 160, 2>;
+    StagedKernel fn = odd ? convection_staged_kernel<3, CG_MAXT, 1, true>
+                          : convection_staged_kernel<6, CG_MAXT, 1>;
+    if (!odd && P * R < 1200 && s.threads <= 160) fn = convection_staged_kernel<3, 160, 2>;
 #endif
     allow_max_dynamic_smem((const void*)fn);
     return fn;
@@ -838,12 +892,18 @@ int VERB_STAGED(conv_staged_ctas)(int P, int R, long long slices)
     return (int)std::min(sms * per, slices);
 }
 
+// The contracted form's second launch finds no slice as a rule (48 x 101 x 101 x 16 23.44
+// ms with it, 23.38 without; 24 x 25 x 31 x 31 1.059 and 1.054 a pass of three runs); its
+// faces in the first one, behind a branch, cost 5 and 3 %.
 void VERB_STAGED(launch_convection_staged)(const ConvArgs& a, int nctas, cudaStream_t st)
 {
     StagedShape s;
     cg_shape(a.d.P, a.d.R, (long long)a.d.V * a.d.K, s);
     const StagedKernel fn = cg_kernel(a.d.P, a.d.R, s);
     fn<<<nctas, s.threads, cg_smem(a.d.P, a.d.R), st>>>(a, s.segP, s.segR);
+#ifndef VERB_BUILD_CONV_EXACT
+    cg_kernel(a.d.P, a.d.R, s, true)<<<nctas, s.threads, cg_smem(a.d.P, a.d.R), st>>>(a, s.segP, s.segR);
+#endif
 }
 
 }  // namespace verb

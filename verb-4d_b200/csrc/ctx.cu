@@ -549,7 +549,7 @@ int conv_run(verb_ctx* c, double dt)
     }
     CK(alloc((void**)&c->conv_scratch, c->conv_scratch_bytes));
     CK(alloc((void**)&c->conv_substeps, (size_t)d.V * d.K * sizeof(int)));
-    CK(alloc((void**)&c->ticket, sizeof(int)));
+    CK(alloc((void**)&c->ticket, (3 + (size_t)d.V * d.K) * sizeof(int)));
     ConvArgs a{};
     a.d = d;
     a.psd = c->f[VERB_F_PSD];
@@ -572,9 +572,10 @@ int conv_run(verb_ctx* c, double dt)
     a.scratch = c->conv_scratch;
     a.substeps = c->conv_substeps;
     a.ticket = c->ticket;
+    a.odd = c->ticket + 3;
     a.status = c->status;
     PhaseTimer t(c, PH_CONV);
-    CK(cudaMemsetAsync(c->ticket, 0, sizeof(int), c->stream));
+    CK(cudaMemsetAsync(c->ticket, 0, 3 * sizeof(int), c->stream));
     if (kernel == VERB_CONV_KERNEL_STAGED && c->conv_arith == VERB_CONV_EXACT)
         launch_convection_staged_exact(a, conv_staged_ctas_exact(d.P, d.R, slices), c->stream);
     else if (kernel == VERB_CONV_KERNEL_STAGED)
@@ -585,7 +586,7 @@ int conv_run(verb_ctx* c, double dt)
         launch_convection(a, c->conv_nctas, c->stream);
     else
         launch_convection_fma(a, c->conv_nctas, c->stream);
-    c->acc.kernel_launches++;
+    c->acc.kernel_launches += kernel == VERB_CONV_KERNEL_STAGED && c->conv_arith == VERB_CONV_STREAM ? 2 : 1;
     return check_launch();
 }
 

@@ -106,7 +106,9 @@ struct ConvArgs {
     double dt;
     double* scratch;     // per-CTA conv_scratch_doubles(P, R): Courant tables and planes
     int* substeps;       // [V][K] out
-    int* ticket;         // work counter (zeroed before launch)
+    int* ticket;         // work counter (zeroed before launch; the contracted two-stage
+                         // form: three, the other two for its second launch)
+    int* odd;            // [V*K] slices left to that launch
     int* status;
 };
 int conv_ctas(int P, int R);
