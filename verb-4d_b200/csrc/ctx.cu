@@ -503,6 +503,9 @@ size_t conv_scratch_size(const Dims& d)
     return b * sizeof(double);
 }
 
+// a sweep of 3 to 10 points (its stencils need 11)
+bool conv_grid_bad(const Dims& d) { return (d.P >= 3 && d.P < 11) || (d.R >= 3 && d.R < 11); }
+
 // The kernel of a convection pass (VERB_CONV_KERNEL_*): the two-stage one where
 // both sweeps run, a slice's planes fit the shared memory and it is the faster
 // (cg_faster); other shapes take one thread per line (stream mode) or the
@@ -510,6 +513,7 @@ size_t conv_scratch_size(const Dims& d)
 int conv_kernel_for(const verb_ctx* c, int& kernel)
 {
     const Dims& d = c->d;
+    if (conv_grid_bad(d)) return VERB_ERR_GRID;
     const long long slices = (long long)d.V * d.K;
     const bool staged = c->conv_arith == VERB_CONV_STREAM ? conv_staged_check(d.P, d.R, slices) == VERB_OK
                         : c->conv_arith == VERB_CONV_EXACT
@@ -524,7 +528,7 @@ int conv_kernel_for(const verb_ctx* c, int& kernel)
 int conv_run(verb_ctx* c, double dt)
 {
     const Dims& d = c->d;
-    if ((d.P >= 3 && d.P < 11) || (d.R >= 3 && d.R < 11)) return VERB_ERR_GRID;
+    if (conv_grid_bad(d)) return VERB_ERR_GRID;
     const bool pper = c->bct[VERB_BCF_PL] == VERB_BC_PERIODIC;
     if (pper != (c->bct[VERB_BCF_PU] == VERB_BC_PERIODIC)) return VERB_ERR_BC;
     const bool rper = c->bct[VERB_BCF_RL] == VERB_BC_PERIODIC;
