@@ -28,21 +28,12 @@
 // whole calls: 3.0 -> 0.81 ms (with the operands in a global workspace, scalar
 // tiles, one thread forming the operator and the observation list, and the
 // observations of every MLT copied to the device).
+#include "dmma.cuh"
 #include "verb_internal.cuh"
 
 namespace verb {
 
 namespace {
-
-// c (8 x 8: row lane / 4, columns 2 (lane % 4), + 1) += a (8 x 4: row lane / 4,
-// column lane % 4) times b (4 x 8: row lane % 4, column lane / 4), the four
-// products added in ascending order, one fused multiply-add each
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b)
-{
-    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-        : "+d"(c[0]), "+d"(c[1])
-        : "d"(a), "d"(b));
-}
 
 constexpr int KF_K4 = 32;  // k steps of four: R <= 128
 
@@ -68,7 +59,7 @@ __device__ __forceinline__ void kf_product(int n, const double* A, int lda, int 
         const double* ar = A + (size_t)(8 * r + g) * lda + h;
 #pragma unroll
         for (int k = 0; k < KF_K4; k++)
-            if (k < nk) dmma(c, ar[4 * k], b[k]);
+            if (k < nk) dmma(c[0], c[1], ar[4 * k], b[k]);
         store(8 * r + g, 8 * w + 2 * h, c);
     }
 }

@@ -21,6 +21,7 @@
 // per-slice exponents (slices whose bit is clear sit out the product); the
 // gain solves run one CTA per slice (LU with partial pivoting of the m x m
 // innovation covariance, the rows of Pf H^T as right-hand sides).
+#include "dmma.cuh"
 #include "verb_internal.cuh"
 
 namespace verb {
@@ -30,16 +31,6 @@ namespace {
 constexpr int BT = 64;   // output tile
 constexpr int BK = 16;   // k step
 constexpr int GT = 128;  // threads: four warps of 32 x 32 outputs
-
-// c (8 x 8: row lane / 4, columns 2 (lane % 4), + 1) += a (8 x 4: row lane / 4,
-// column lane % 4) times b (4 x 8: row lane % 4, column lane / 4), the four
-// products added in ascending order, one fused multiply-add each
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b)
-{
-    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-        : "+d"(c[0]), "+d"(c[1])
-        : "d"(a), "d"(b));
-}
 
 // C = Cin + sgn * (A diag(dk) op(B)), or A diag(dk) op(B) when Cin is null.
 // A: M x K (lda), B: K x N (ldb) or, with TB, N x K; batch b -> slice
@@ -134,7 +125,7 @@ __global__ void __launch_bounds__(GT, 3) bgemm_kernel(BGemm g)
 #pragma unroll
             for (int r = 0; r < 4; r++)
 #pragma unroll
-                for (int c = 0; c < 4; c++) dmma(acc[r][c], a[r], b[c]);
+                for (int c = 0; c < 4; c++) dmma(acc[r][c][0], acc[r][c][1], a[r], b[c]);
         }
         p = p + 1 == GS ? 0 : p + 1;
     }

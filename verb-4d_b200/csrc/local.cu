@@ -39,6 +39,7 @@
 // -fmad=false) except the factorisation's rank-1 update, which both compute
 // as one fused multiply-add per element (fma()), so factors, pivots and
 // solutions are bit-identical to it.
+#include "dmma.cuh"
 #include "exact_div.cuh"
 #include "verb_internal.cuh"
 
@@ -449,15 +450,6 @@ __device__ __forceinline__ void named_sync(int id, int threads)
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// c (8 x 8: row lane / 4, columns 2 (lane % 4), + 1) += a (8 x 4: row lane / 4,
-// column lane % 4) times b (4 x 8: row lane % 4, column lane / 4)
-__device__ __forceinline__ void dmma(double2& c, double a, double b)
-{
-    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-        : "+d"(c.x), "+d"(c.y)
-        : "d"(a), "d"(b));
-}
-
 // *p = (x, y) in shared memory where c holds, as a predicated store
 __device__ __forceinline__ void sts2_if(bool c, double* p, double x, double y)
 {
@@ -860,7 +852,7 @@ __global__ void __launch_bounds__(NW * 32, fb_min_blocks(PW)) local_factor_blk_k
 #pragma unroll
                         for (int e = 0; e < 2; e++)
 #pragma unroll
-                            for (int i = 0; i < 2; i++) dmma(acc[i][e], l[i][k], u[e][k]);
+                            for (int i = 0; i < 2; i++) dmma(acc[i][e].x, acc[i][e].y, l[i][k], u[e][k]);
 #pragma unroll
                     for (int e = 0; e < 2; e++)
 #pragma unroll
