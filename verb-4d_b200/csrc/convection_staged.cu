@@ -130,6 +130,12 @@ __device__ __forceinline__ void line_ghosts(double* E, int st, int n, int lt, in
 // polynomials and the limiters of a group are independent of each other, and
 // the window is loaded once per group instead of shifted through registers.
 
+// NaN, infinite or above 2^300
+__device__ __forceinline__ bool is_odd(double v)
+{
+    return ((unsigned)__double2hiint(v) & 0x7fffffffu) >= 0x52b00000u;
+}
+
 // Unlimited value of one face from its stencil e[k * st] = E[x-5+k], the
 // reference's sums as they stand
 __device__ __forceinline__ double face_alone(const double* e, int st, double c)
@@ -222,11 +228,6 @@ __device__ __forceinline__ void faces(double (&d)[U + 9], const double (&c)[U], 
         f[u] += (p[u] * (1.0 / 362880.0)) * (c[u] >= 0 ? d[u] : d[u + 1]);
 }
 
-// NaN, infinite or above 2^300
-__device__ __forceinline__ bool is_odd(double v)
-{
-    return ((unsigned)__double2hiint(v) & 0x7fffffffu) >= 0x52b00000u;
-}
 #endif
 
 // returns unlimited face a, whose slot is the neighbour's
@@ -578,7 +579,7 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
 #else
             const double eg = exp(a.loss[gi] * dtc) / G;
             e1R[(size_t)iR * P + iP] = eg;
-            if (is_odd(S[iP * Rs + iR]) || is_odd(G) || is_odd(eg) || is_odd(a.S[gi])) odd = true;
+            odd |= is_odd(S[iP * Rs + iR]) || is_odd(G) || is_odd(eg) || is_odd(a.S[gi]);
 #endif
             e2R[(size_t)iR * P + iP] = iR && iR < R - 1 ? a.S[gi] * dtc : -0.0;
         }
@@ -621,22 +622,20 @@ __global__ void __launch_bounds__(MAXT, MINB) convection_staged_kernel(ConvArgs 
             line_table(a.VP, a.Pg, iR, P, true, crP, rcP, nsP, lnP, R - 1);
             if (lane == 0) {
                 const size_t bo = ((size_t)iR * V + iV) * K + iK;
-                lnP[iR] = a.Pl[bo];
-                lnP[(R - 1) + iR] = a.Pu[bo];
-#ifndef VERB_BUILD_CONV_EXACT
-                if (a.Pl_t != VERB_BC_PERIODIC && (is_odd(a.Pl[bo]) || is_odd(a.Pu[bo]))) odd = true;
-#endif
+                const double lb = a.Pl[bo], ub = a.Pu[bo];
+                lnP[iR] = lb;
+                lnP[(R - 1) + iR] = ub;
+                odd |= a.Pl_t != VERB_BC_PERIODIC && (is_odd(lb) || is_odd(ub));
             }
         }
         for (int iP = warp; iP < P; iP += nw) {
             line_table(a.VR, a.Rg, iP, R, false, crR, rcR, nsR, lnR, P);
             if (lane == 0) {
                 const size_t bo = ((size_t)iP * V + iV) * K + iK;
-                lnR[iP] = a.Rl[bo] * a.G[g(iP, 0)];
-                lnR[P + iP] = a.Ru[bo] * a.G[g(iP, R - 1)];
-#ifndef VERB_BUILD_CONV_EXACT
-                if (a.Rl_t != VERB_BC_PERIODIC && (is_odd(lnR[iP]) || is_odd(lnR[P + iP]))) odd = true;
-#endif
+                const double lb = a.Rl[bo] * a.G[g(iP, 0)], ub = a.Ru[bo] * a.G[g(iP, R - 1)];
+                lnR[iP] = lb;
+                lnR[P + iP] = ub;
+                odd |= a.Rl_t != VERB_BC_PERIODIC && (is_odd(lb) || is_odd(ub));
             }
         }
         double steps = num_steps;
@@ -793,14 +792,18 @@ int cg_own(int P, int R, long long) { return P * R < 1200 ? 5 : 11; }
 constexpr int CG_STEP = 6;
 #endif
 
+void cg_segments(int P, int R, int own, StagedShape& s)
+{
+    s.own = own;
+    s.segP = (P - 1 + own - 1) / own;
+    s.segR = (R - 1 + own - 1) / own;
+    s.threads = (std::max((R - 1) * s.segP, P * s.segR) + 31) / 32 * 32;
+}
+
 bool cg_shape(int P, int R, long long slices, StagedShape& s)
 {
     for (int own = cg_own(P, R, slices); own <= CG_MAX_OWN; own += CG_STEP) {
-        s.own = own;
-        s.segP = (P - 1 + own - 1) / own;
-        s.segR = (R - 1 + own - 1) / own;
-        const int need = std::max((R - 1) * s.segP, P * s.segR);
-        s.threads = (need + 31) / 32 * 32;
+        cg_segments(P, R, own, s);
         if (s.threads <= CG_MAXT) return true;
     }
     return false;
@@ -814,9 +817,10 @@ StagedKernel cg_kernel(int P, int R, const StagedShape& s, bool odd = false)
     if (s.threads <= 320) fn = convection_staged_kernel<3, 320, 1>;
     if (s.threads <= 160) fn = convection_staged_kernel<3, 160, 2>;
 #else
-    StagedKernel fn = odd ? convection_staged_kernel<3, CG_MAXT, 1, true>
+    StagedKernel fn = odd ? convection_staged_kernel<6, CG_MAXT, 1, true>
                           : convection_staged_kernel<6, CG_MAXT, 1>;
-    if (!odd && P * R < 1200 && s.threads <= 160) fn = convection_staged_kernel<3, 160, 2>;
+    if (P * R < 1200 && s.threads <= 160)
+        fn = odd ? convection_staged_kernel<3, 160, 2, true> : convection_staged_kernel<3, 160, 2>;
 #endif
     allow_max_dynamic_smem((const void*)fn);
     return fn;
@@ -892,9 +896,11 @@ int VERB_STAGED(conv_staged_ctas)(int P, int R, long long slices)
     return (int)std::min(sms * per, slices);
 }
 
-// The contracted form's second launch finds no slice as a rule (48 x 101 x 101 x 16 23.44
-// ms with it, 23.38 without; 24 x 25 x 31 x 31 1.059 and 1.054 a pass of three runs); its
-// faces in the first one, behind a branch, cost 5 and 3 %.
+// The contracted form's second launch finds no slice as a rule.  Three runs at once,
+// without it and with it: 48 x 101 x 101 x 16 23.38 -> 23.44 ms a pass, 24 x 25 x 31 x 31 1.066
+// -> 1.067, 42 x 15 x 20 x 8 1.38 -> 1.41, 12 x 13 x 31 x 31 0.436 -> 0.451 (it waits behind the
+// other streams' blocks).  Its faces in the first launch, behind a branch, cost 5 % at
+// 48 x 101 x 101 x 16 and 3 % at 24 x 25 x 31 x 31; a call for the whole slice there 1 to 5 %.
 void VERB_STAGED(launch_convection_staged)(const ConvArgs& a, int nctas, cudaStream_t st)
 {
     StagedShape s;
@@ -902,7 +908,10 @@ void VERB_STAGED(launch_convection_staged)(const ConvArgs& a, int nctas, cudaStr
     const StagedKernel fn = cg_kernel(a.d.P, a.d.R, s);
     fn<<<nctas, s.threads, cg_smem(a.d.P, a.d.R), st>>>(a, s.segP, s.segR);
 #ifndef VERB_BUILD_CONV_EXACT
-    cg_kernel(a.d.P, a.d.R, s, true)<<<nctas, s.threads, cg_smem(a.d.P, a.d.R), st>>>(a, s.segP, s.segR);
+    // (few blocks, of the same shape as the first launch's: another split of an SM's
+    // shared memory would have to wait for other streams' blocks to leave it)
+    cg_kernel(a.d.P, a.d.R, s, true)<<<std::min(nctas, 16), s.threads, cg_smem(a.d.P, a.d.R), st>>>(
+        a, s.segP, s.segR);
 #endif
 }
 
